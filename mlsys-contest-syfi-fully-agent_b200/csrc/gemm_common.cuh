@@ -34,6 +34,28 @@ struct Aux {
 };
 static_assert(sizeof(Aux) <= 1024, "Aux must fit its slot");
 
+// The schedule as every warp of the grouped GEMM kernels keeps it: lane = local expert.  An item index is decoded with
+// one ballot and four shuffles; a binary search through shared memory is five dependent loads, and a role pays
+// for it once per item, between two items' loads, UMMAs or promotions.
+struct LaneSched {
+  int pfx, tiles, off, cnt;
+  __device__ __forceinline__ void load(const int* tile_prefix, const int* offs, int lane) {
+    pfx = __ldcg(tile_prefix + lane);
+    tiles = __ldcg(tile_prefix + lane + 1) - pfx;
+    off = __ldcg(offs + lane);
+    cnt = __ldcg(offs + lane + 1) - off;
+  }
+  // Expert that owns item i when a token tile has `per` items: the largest e with pfx[e] * per <= i (experts without
+  // tiles repeat the prefix, so the largest such e has tiles).  r = item inside the expert.
+  __device__ __forceinline__ void find(int i, int per, int& e, unsigned& r, unsigned& tiles_e, int& off_e, int& cnt_e) const {
+    e = __popc(__ballot_sync(0xFFFFFFFFu, pfx * per <= i)) - 1;
+    r = static_cast<unsigned>(i - __shfl_sync(0xFFFFFFFFu, pfx, e) * per);
+    tiles_e = static_cast<unsigned>(__shfl_sync(0xFFFFFFFFu, tiles, e));
+    off_e = __shfl_sync(0xFFFFFFFFu, off, e);
+    cnt_e = __shfl_sync(0xFFFFFFFFu, cnt, e);
+  }
+};
+
 // Extra shared state of the decode-fused kernels: every CTA routes all (<= 16) tokens itself.
 struct FusedAux {
   float sval[kEGlobal];               // routing bias as fp32

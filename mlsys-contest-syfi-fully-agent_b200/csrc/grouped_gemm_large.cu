@@ -112,18 +112,6 @@ __device__ __forceinline__ LItem decode_large(int i, const LAux* aux) {
   return it;
 }
 
-// acc[0..32) += v[0..32) * f with the packed two-element fp32 FMA of sm_100 (each element is one IEEE fma, the
-// same result as fmaf): half the instructions of the scalar form, and the promotion warps are issue-bound.
-__device__ __forceinline__ void fma32(float* acc, const float* v, float f) {
-  const float2 ff = make_float2(f, f);
-#pragma unroll
-  for (int x = 0; x < 16; ++x) {
-    const float2 r = __ffma2_rn(make_float2(v[2 * x], v[2 * x + 1]), ff, make_float2(acc[2 * x], acc[2 * x + 1]));
-    acc[2 * x] = r.x;
-    acc[2 * x + 1] = r.y;
-  }
-}
-
 __device__ __forceinline__ void red_add_v4(float* p, float x, float y, float z, float w) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
@@ -262,7 +250,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       const int lrow = min(row, a.rows_cap - 1);   // rows past the tile's last one are computed and dropped
       if constexpr (GEMM == 1) {
         // scales of this thread's token row and of the item's two weight blocks, read one K-block ahead
-        const float* bsp = a.b_scale + static_cast<size_t>(lrow) * kKB1;
+        const float* bsp = a.b_scale + lrow;   // [56][rows_cap]: a warp's 32 rows are one line
         const float* w1p = a.w_scale + (static_cast<size_t>(w.e) * kMT1 + w.j) * kKB1;
         const float* w2p = w1p + kKB2 * kKB1;   // the block 16 further: the second half of W13
         float acc[64];      // [0, 32): x1 of this thread's 32 columns, [32, 64): x2 of the same columns
@@ -278,15 +266,15 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
           tmem_ld32(taddr, v);                  // x1: columns cg*32 .. +32 of the first 128
           // (scale arithmetic and the next K-block's scale loads run under the read-back's latency)
           const float f1 = n1 * nb, f2 = n2 * nb;
-          if (s + 1 < kKB1) { nb = __ldg(bsp + s + 1); n1 = __ldg(w1p + s + 1); n2 = __ldg(w2p + s + 1); }
+          if (s + 1 < kKB1) { nb = __ldg(bsp + static_cast<size_t>(s + 1) * a.rows_cap); n1 = __ldg(w1p + s + 1); n2 = __ldg(w2p + s + 1); }
           tmem_wait_ld();
-          fma32(acc, v, f1);
+          fma_scaled<32>(acc, v, f1);
           tmem_ld32(taddr + 128, v);            // x2: the same columns of the second 128
           tmem_wait_ld();
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(tempty_base + buf * 8);
-          fma32(acc + 32, v, f2);
+          fma_scaled<32>(acc + 32, v, f2);
           if (++stage == C::STAGES) { stage = 0; ph ^= 1u; }
           if (++buf == C::NBUF) { buf = 0; bph ^= 1u; }
         }
@@ -321,12 +309,16 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
             dst[0] = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
             dst[1] = make_uint4(pk[t][4], pk[t][5], pk[t][6], pk[t][7]);
           }
-          if (cg == 0) a.c_scale[static_cast<size_t>(row) * kKB2 + w.j] = __uint_as_float(static_cast<uint32_t>(ex + 127) << 23);
+          if (cg == 0) {
+            const float scale = __uint_as_float(static_cast<uint32_t>(ex + 127) << 23);
+            a.c_scale[static_cast<size_t>(row) * kKB2 + w.j] = scale;
+            a.c_scale_kb[static_cast<size_t>(w.j) * a.rows_cap + row] = scale;
+          }
         }
       } else {
         // this thread's 64 columns lie in ONE 128-row weight block: 2 j + (cg >> 1)
         const int tile = 2 * w.j + (cg >> 1);
-        const float* bsp = a.b_scale + static_cast<size_t>(lrow) * kKB2;
+        const float* bsp = a.b_scale + lrow;   // [16][rows_cap]
         const float* wsp = a.w_scale + (static_cast<size_t>(w.e) * kMT2 + tile) * kKB2;
         float acc[64];
 #pragma unroll
@@ -340,15 +332,15 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
           float v[32];
           tmem_ld32(taddr, v);
           const float f = nw * nb;
-          if (s + 1 < kKB2) { nb = __ldg(bsp + s + 1); nw = __ldg(wsp + s + 1); }
+          if (s + 1 < kKB2) { nb = __ldg(bsp + static_cast<size_t>(s + 1) * a.rows_cap); nw = __ldg(wsp + s + 1); }
           tmem_wait_ld();
-          fma32(acc, v, f);
+          fma_scaled<32>(acc, v, f);
           tmem_ld32(taddr + 32, v);
           tmem_wait_ld();
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(tempty_base + buf * 8);
-          fma32(acc + 32, v, f);
+          fma_scaled<32>(acc + 32, v, f);
           if (++stage == C::STAGES) { stage = 0; ph ^= 1u; }
           if (++buf == C::NBUF) { buf = 0; bph ^= 1u; }
         }

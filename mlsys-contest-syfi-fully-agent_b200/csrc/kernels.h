@@ -73,7 +73,8 @@ struct GatherArgs {
   const float* hidden_scale;    // [56, T]
   int T;
   uint8_t* a_packed;            // [rows_cap, 7168]
-  float* a_scale_rows;          // [rows_cap, 56] scales of each permuted row, row-major
+  int rows_cap;
+  float* a_scale;               // [56, rows_cap] scales of the permuted rows, K-block-major (a warp's rows are adjacent)
 };
 
 // Grouped, swap-AB, split-K fp8 GEMM: out[slab][row, m] = sum_k W_e[m, k] * B[row, k] with the
@@ -82,7 +83,7 @@ struct GatherArgs {
 struct GemmArgs {
   MoeSched* sched;
   const float* w_scale;         // [32, M/128, K/128]
-  const float* b_scale;         // per-row scales, row-major: GEMM1 [rows, 56]; GEMM2 [rows, 16]
+  const float* b_scale;         // scales of the rows, K-block-major: GEMM1 [56, rows_cap]; GEMM2 [16, rows_cap]
   float* out;                   // fp32 slabs [split][n_sel_pad, M]
   // ---- only read by the single-launch decode kernel (T <= 16), see decode_kernel.cu
   const float* logits;          // [T, 256]
@@ -93,7 +94,8 @@ struct GemmArgs {
   int ctas, rows_cap, slab_rows;
   int* topk_idx; float* topk_w; uint32_t* local_mask;
   int* perm_token; float* perm_weight; int* tok_rows;
-  uint8_t* cq; float* c_scale;  // SwiGLU planes and their scales
+  uint8_t* cq; float* c_scale;  // SwiGLU planes and their scales [rows_cap, 16]
+  float* c_scale_kb;            // the scales again as [16, rows_cap] (GEMM2's b_scale); null in the decode kernel
   uint16_t* out_bf16;           // final output
   uint16_t* const* out_rows;    // optional per-token destinations instead of out_bf16 (may be peer memory)
   // ---- only read by the large-batch GEMM2 with the fused combine (grouped_gemm_large.cu)
@@ -106,6 +108,7 @@ struct SwigluArgs {
   const float* g1;              // slabs [split1][n_sel_pad, 4096]
   uint8_t* cq;                  // [kNTerms][rows_cap, 2048] e4m3 planes
   float* c_scale;               // [rows_cap, 16] power-of-two plane scale per 128 block
+  float* c_scale_kb;            // the same, [16, rows_cap]
   int rows_cap;
 };
 
@@ -129,14 +132,14 @@ int route_permute_launches(int T);   // kernels launch_route_permute starts for 
 void launch_route_permute(const RouteArgs& r, const PermuteArgs& p, cudaStream_t stream);
 void launch_route_only(const RouteArgs& r, cudaStream_t stream);
 void launch_gather_rows(const GatherArgs& a, int T, cudaStream_t stream);
-// gemm_id 1 or 2; n_tile in {16, 32, 64, 128}.  Returns a cudaError_t as int.
+// gemm_id 1 or 2; n_tile in {32, 64, 128}.  Returns a cudaError_t as int.
 // Token-operand tensor maps of grouped_gemm_kernel: the same tensor with boxes of 1..4 row steps
-// (grouped_gemm_row_step(n_tile) rows each), so that a token tile with few valid rows (the last tile of an
+// (32 rows each), so that a token tile with few valid rows (the last tile of an
 // expert, or an expert with a handful of tokens) brings only the rows it has, rounded up to a step.
 struct TokenMaps {
   CUtensorMap m[4];
 };
-int grouped_gemm_row_step(int n_tile);   // rows per step: n_tile / 4 from 64-token tiles up, else 16
+int grouped_gemm_row_step(int n_tile);
 int launch_grouped_gemm(int gemm_id, int n_tile, const CUtensorMap& tm_w, const TokenMaps& tm_b, const GemmArgs& a,
                         int ctas, cudaStream_t stream);
 constexpr int kFusedMaxTokens = 16;

@@ -282,10 +282,11 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
   int* tok_rows = reinterpret_cast<int*>(ws + L.tok_rows);
   int* chunk_base = reinterpret_cast<int*>(ws + L.chunk_base);
   uint8_t* a_packed = ws + L.a_packed;
-  float* a_scale_rows = reinterpret_cast<float*>(ws + L.a_scale_rows);
+  float* a_scale = reinterpret_cast<float*>(ws + L.a_scale_rows);
   float* g1 = reinterpret_cast<float*>(ws + L.g1);
   uint8_t* cq = ws + L.cq;
   float* c_scale = reinterpret_cast<float*>(ws + L.c_scale);
+  float* c_scale_kb = reinterpret_cast<float*>(ws + L.c_scale_kb);
   float* o = reinterpret_cast<float*>(ws + L.o);
   float* acc32 = reinterpret_cast<float*>(ws + L.acc32);
   int* tile_cnt = reinterpret_cast<int*>(ws + L.tile_cnt);
@@ -347,17 +348,17 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
   g_launches += route_permute_launches(T);
   stage_mark(1, stream);
 
-  GatherArgs ga{sched, perm_token, hidden_states, hidden_states_scale, T, a_packed, a_scale_rows};
+  GatherArgs ga{sched, perm_token, hidden_states, hidden_states_scale, T, a_packed, L.rows_cap, a_scale};
   launch_gather_rows(ga, T, stream);
   MOE_CUDA(cudaGetLastError());
   g_launches += 1;
   stage_mark(2, stream);
 
   GemmArgs g1a{};
-  g1a.sched = sched; g1a.w_scale = gemm1_weights_scale; g1a.b_scale = a_scale_rows; g1a.out = g1;
-  g1a.rows_cap = L.rows_cap; g1a.cq = cq; g1a.c_scale = c_scale;
+  g1a.sched = sched; g1a.w_scale = gemm1_weights_scale; g1a.b_scale = a_scale; g1a.out = g1;
+  g1a.rows_cap = L.rows_cap; g1a.cq = cq; g1a.c_scale = c_scale; g1a.c_scale_kb = c_scale_kb;
   GemmArgs g2a{};
-  g2a.sched = sched; g2a.w_scale = gemm2_weights_scale; g2a.b_scale = c_scale; g2a.out = o;
+  g2a.sched = sched; g2a.w_scale = gemm2_weights_scale; g2a.b_scale = c_scale_kb; g2a.out = o;
   g2a.rows_cap = L.rows_cap; g2a.perm_token = perm_token; g2a.perm_weight = perm_weight; g2a.local_mask = local_mask;
   g2a.acc32 = acc32; g2a.tile_cnt = tile_cnt; g2a.out_bf16 = output; g2a.out_rows = output_rows;
 
@@ -401,7 +402,7 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
     g_launches += 1;
     stage_mark(3, stream);
 
-    SwigluArgs sa{sched, g1, cq, c_scale, L.rows_cap};
+    SwigluArgs sa{sched, g1, cq, c_scale, c_scale_kb, L.rows_cap};
     launch_swiglu_split(sa, T, stream);
     MOE_CUDA(cudaGetLastError());
     g_launches += 1;

@@ -26,6 +26,22 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
+// One lane of a converged warp, always the same one.  Around tcgen05 and TMA instructions this and not `lane == 0`:
+// the compiler knows that exactly one lane takes the branch and feeds the instructions from uniform registers, while
+// under `lane == 0` it wraps each of them in a loop over the active lanes (four UMMAs and a commit: 430 clocks of
+// issue against 200, whatever the UMMAs' size).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+// The warp's index as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0); }
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -66,18 +82,30 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // next poll and leave too.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   uint32_t spins = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
     if ((++spins & 0x3Fu) == 0) {
-      if (globaltimer_ns() - t0 > MOE_WAIT_LIMIT_NS) {
+      const uint64_t t = globaltimer_ns();
+      if (t0 == 0) t0 = t;
+      else if (t - t0 > MOE_WAIT_LIMIT_NS) {
         *abort_flag = 1;
         return false;
       }
     }
   }
+}
+
+// ----------------------------------------------------------------------------- cp.async (4 bytes per thread)
+// Asynchronous copy global -> shared memory; `cp_async_arrive` makes the mbarrier phase wait for all of the calling
+// thread's earlier copies (one ordinary arrival, counted in the barrier's init count, when they have landed).
+__device__ __forceinline__ void cp_async4(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // ----------------------------------------------------------------------------- TMA (tiled, no multicast)
@@ -227,11 +255,33 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
       : "memory");
 }
 
+// Waits for this thread's TMEM reads and ties the 32 registers of one to the wait, so that the compiler cannot
+// move their use in front of it when other work stands between the read and the wait.
+__device__ __forceinline__ void tmem_wait_ld32(float* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31])
+               :
+               : "memory");
+}
+
 // 32-byte store (a full DRAM sector) of eight consecutive floats; the address must be 32-byte aligned.
 __device__ __forceinline__ void st_global_v8(float* p, const float* v) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                : "memory");
+}
+
+// acc[0..N) += v[0..N) * f with the packed two-element fp32 FMA of sm_100 (each element is one IEEE fma, the
+// same result as fmaf): half the instructions of the scalar form.
+template <int N>
+__device__ __forceinline__ void fma_scaled(float* acc, const float* v, float f) {
+  const float2 ff = make_float2(f, f);
+#pragma unroll
+  for (int x = 0; x < N / 2; ++x) {
+    const float2 r = __ffma2_rn(make_float2(v[2 * x], v[2 * x + 1]), ff, make_float2(acc[2 * x], acc[2 * x + 1]));
+    acc[2 * x] = r.x;
+    acc[2 * x + 1] = r.y;
+  }
 }
 
 // Register reallocation between warpgroups (each executed by all four warps of a warpgroup).

@@ -305,31 +305,26 @@ __global__ void __launch_bounds__(1024) route_permute_kernel(RouteArgs r, Permut
 }
 
 // Packed copy of the fp8 activation rows in permuted order: a_packed[r, :] = hidden[perm_token[r], :]
-// (the B operand of GEMM1 is then one TMA box per token tile), 16 bytes per thread, plus the
-// row's 56 block scales gathered from the transposed [56, T] layout into a row-major table.
+// (the B operand of GEMM1 is then one TMA box per token tile), 16 bytes per thread, plus the rows' block
+// scales as [56, rows_cap]: the GEMMs' promotion threads own one row each, so a warp's scales of a K-block
+// are one line here, and were 32 lines in a row-major table.
 __global__ void __launch_bounds__(256) gather_rows_kernel(GatherArgs a) {
   griddep_launch_dependents();
   griddep_wait();
   const int n_sel = a.sched->n_sel;
   constexpr int kData = kH / 16;            // 448 x 16 B of fp8 per row
-  constexpr int kChunks = kData + kKB1 / 4; // + 14 x 4 scales
-  const long long total = static_cast<long long>(n_sel) * kChunks;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int r = static_cast<int>(i / kChunks), c = static_cast<int>(i % kChunks);
+  const long long total = static_cast<long long>(n_sel) * kData;
+  const long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = first; i < total; i += stride) {
+    const int r = static_cast<int>(i / kData), c = static_cast<int>(i % kData);
     const int t = a.perm_token[r];
-    if (c < kData) {
-      reinterpret_cast<uint4*>(a.a_packed + static_cast<size_t>(r) * kH)[c] =
-          __ldg(reinterpret_cast<const uint4*>(a.hidden + static_cast<size_t>(t) * kH) + c);
-    } else {
-      const int kb = (c - kData) * 4;
-      float4 v;
-      v.x = __ldg(a.hidden_scale + static_cast<size_t>(kb + 0) * a.T + t);
-      v.y = __ldg(a.hidden_scale + static_cast<size_t>(kb + 1) * a.T + t);
-      v.z = __ldg(a.hidden_scale + static_cast<size_t>(kb + 2) * a.T + t);
-      v.w = __ldg(a.hidden_scale + static_cast<size_t>(kb + 3) * a.T + t);
-      reinterpret_cast<float4*>(a.a_scale_rows + static_cast<size_t>(r) * kKB1)[c - kData] = v;
-    }
+    reinterpret_cast<uint4*>(a.a_packed + static_cast<size_t>(r) * kH)[c] =
+        __ldg(reinterpret_cast<const uint4*>(a.hidden + static_cast<size_t>(t) * kH) + c);
+  }
+  for (long long i = first; i < static_cast<long long>(n_sel) * kKB1; i += stride) {
+    const int kb = static_cast<int>(i / n_sel), r = static_cast<int>(i % n_sel);
+    a.a_scale[static_cast<size_t>(kb) * a.rows_cap + r] = __ldg(a.hidden_scale + static_cast<size_t>(kb) * a.T + a.perm_token[r]);
   }
 }
 
@@ -356,7 +351,7 @@ void launch_route_only(const RouteArgs& r, cudaStream_t stream) {
 }
 
 void launch_gather_rows(const GatherArgs& a, int T, cudaStream_t stream) {
-  long long chunks = static_cast<long long>(T) * kTopK * (kH / 16 + kKB1 / 4);
+  long long chunks = static_cast<long long>(T) * kTopK * (kH / 16);
   long long blocks = (chunks + 255) / 256;
   if (blocks > 8 * kNumSMs) blocks = 8 * kNumSMs;
   if (blocks < 1) blocks = 1;
