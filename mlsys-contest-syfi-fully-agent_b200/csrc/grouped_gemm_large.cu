@@ -28,12 +28,20 @@
 // FMA per element (they cannot ride on the hardware's power-of-two block scaling).
 //
 // Roles (640 threads, one CTA per SM):
-//   warp 0      TMA producer (one thread; SWIZZLE_128B boxes, no multicast)
-//   warps 1, 2  UMMA issuers (one thread each, alternate pipeline stages)
+//   warp 0      TMA producer (one elected lane; SWIZZLE_128B boxes, no multicast).  Weights and token planes have rings
+//               of their own: a K-block of GEMM2 is 80 KB, two whole ones are all that fits, and then the load of one
+//               is exposed behind the UMMAs of the other; one plane at a time, 2.3 to 3 K-blocks are in flight.  A
+//               ragged token tile brings the rows it has (boxes of 1 to 4 times 32 rows); the rows behind them are
+//               whatever the slot held before, and their lanes of the accumulator are never read.
+//   warps 1, 2  UMMA issuers (one elected lane each, alternate K-blocks)
+//   warp 3      scales of every K-block, copied asynchronously into a ring in shared memory behind the K-block's own
+//               barrier: the promotion warps' loads from global memory were a round trip in every K-block
 //   warps 4-19  promotion + epilogue: four warps per TMEM lane quarter, each owning a quarter of the
 //               accumulator columns.  Sixteen warps (four per scheduler) so that the TMEM read-back
 //               latency of one warp is covered by the FMAs of the others; with eight the read-back
 //               latency was exposed in every K-block and the tensor pipe sat idle two thirds of the time.
+// The two rings, the scale warp, the ragged boxes and the elected lanes together: T = 4096 778 -> 695 us per call,
+// T = 14107 1644 -> 1475 us, the 256-expert layer at T = 16384 15.3 -> 13.9 ms (per call, both builds in turn).
 // Every wait is bounded (ptx.cuh); a timeout raises the CTA's abort flag, all roles fall through to
 // the normal teardown (TMEM freed) and an error bit is left in the schedule block.
 #include "epilogue_device.cuh"
@@ -43,6 +51,7 @@
 namespace moe {
 namespace {
 
+constexpr int kRowStep = kLargeRowStep;
 constexpr int kLEpiWarps = 16;
 constexpr int kLFirstEpi = 4;
 constexpr int kLEpiThreads = kLEpiWarps * 32;
@@ -63,21 +72,37 @@ struct LCfg {
   static constexpr int W_ROWS = 256;                             // weight rows of an item = UMMA N = TMEM columns per K-block
   static constexpr int W_BYTES = W_ROWS * 128;                   // one K-block of the weight operand
   static constexpr int TOK_BYTES = 128 * 128;                    // one K-block of 128 token rows (one plane)
-  static constexpr int STAGE_BYTES = W_BYTES + NTERMS * TOK_BYTES;   // one K-block per pipeline stage: 48 KB / 80 KB
-  static constexpr int STAGES = GEMM == 1 ? 4 : 2;
-  static constexpr int BUF_COLS = W_ROWS;                        // TMEM columns of one stage's partial sums
-  static constexpr int NBUF = 2;                                 // not deeper than the stage ring
+  // Two rings: one K-block of weights per slot, one PLANE of a K-block of tokens per slot.  A slot is free as soon as
+  // the four UMMAs of its plane (weights: of the K-block's last plane) have completed.
+  static constexpr int WS = GEMM == 1 ? 4 : 3;
+  static constexpr int PS = GEMM == 1 ? 4 : 7;
+  static constexpr int BUF_COLS = W_ROWS;                        // TMEM columns of one K-block's partial sums
+  static constexpr int NBUF = 2;
   static constexpr int TMEM_COLS = 512;
+  // Scales of one K-block: 128 row scales, then the two weight scales of the item's 256 weight rows.  A slot is written
+  // again NSLOT K-blocks later; its writer has then seen K-block WS before complete, whose UMMAs waited for the
+  // promotion warps to release the buffer of NBUF before that, after they had read that K-block's scales.
+  static constexpr int SLOT_FLOATS = 128 + 4;
+  static constexpr int NSLOT = WS + NBUF + 1;
+  static constexpr int SLOTS_BYTES = (NSLOT * SLOT_FLOATS * 4 + 127) / 128 * 128;
   static constexpr int AUX_BYTES = 4096;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + AUX_BYTES + 1024;
-  static_assert(NBUF * BUF_COLS <= TMEM_COLS && NBUF <= STAGES, "TMEM ring");
+  static constexpr int RING_BYTES = WS * W_BYTES + PS * TOK_BYTES;
+  static constexpr int SMEM_BYTES = RING_BYTES + SLOTS_BYTES + AUX_BYTES + 1024;
+  static_assert(NBUF * BUF_COLS <= TMEM_COLS, "TMEM ring");
+  // A `pdone` phase must be seen by everybody before its slot's next one completes: the promotion warps are at most
+  // NBUF K-blocks behind the issuers, and the plane that completes the next phase is PS planes later.
+  static_assert(PS >= NBUF * NTERMS && PS >= NTERMS && WS >= NBUF, "ring depths");
+  // The producer waits for K-block n - WS before it loads K-block n's weights, on the barrier of that K-block's last
+  // plane: the next plane on that barrier must not be loaded before, i.e. not belong to an earlier K-block than n.
+  static_assert(NTERMS - 1 + PS >= WS * NTERMS, "a weight slot's barrier must still show the phase that is waited for");
   static_assert(SMEM_BYTES <= 227 * 1024 && SMEM_BYTES > 116 * 1024, "one CTA per SM");
 };
 
 struct LAux {
-  uint64_t full[4];        // TMA -> issuer
-  uint64_t done[4];        // issuer -> producer and promotion warps
-  uint64_t tempty[4];      // promotion warps -> issuer
+  uint64_t wfull[4];       // TMA and the scale warp -> issuers: a K-block's weights (GEMM1: and tokens) and scales
+  uint64_t pfull[8];       // TMA -> issuers: one plane of tokens (GEMM2)
+  uint64_t pdone[8];       // issuers -> producer, scale warp, promotion warps: the UMMAs of a plane have completed
+  uint64_t tempty[2];      // promotion warps -> issuers
   uint64_t esync;          // all promotion threads meet (bounded replacement of a named barrier)
   uint32_t tmem_base;
   int abort;
@@ -86,6 +111,16 @@ struct LAux {
   float amax[4][128];      // per column group and token row: |C| maximum of the thread's columns
 };
 static_assert(sizeof(LAux) <= 4096, "LAux must fit its slot");
+
+// A position in a ring of N slots and the parity of its round.
+template <int N>
+struct Pos {
+  uint32_t i = 0, ph = 0;
+  __device__ __forceinline__ void step(uint32_t k = 1) {
+    i += k;
+    if (i >= N) { i -= N; ph ^= 1u; }
+  }
+};
 
 struct LItem {
   int e, j, row0, valid;
@@ -118,29 +153,31 @@ __device__ __forceinline__ void red_add_v4(float* p, float x, float y, float z, 
 
 template <int GEMM, bool COMBINE>
 __global__ void __launch_bounds__(kLThreads, 1)
-grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b,
+grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ TokenMaps tm_b,
                           const __grid_constant__ GemmArgs a) {
   using C = LCfg<GEMM>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  LAux* aux = reinterpret_cast<LAux*>(smem + C::STAGES * C::STAGE_BYTES);
+  float* slots = reinterpret_cast<float*>(smem + C::RING_BYTES);
+  LAux* aux = reinterpret_cast<LAux*>(smem + C::RING_BYTES + C::SLOTS_BYTES);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   griddep_launch_dependents();
   MoeSched* sched = a.sched;
   // everything that does not depend on earlier kernels first: barriers, descriptors, TMEM
   if (threadIdx.x == 0) {
     aux->abort = 0;
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(smem_u32(&aux->full[s]), 1);
-      mbar_init(smem_u32(&aux->done[s]), 1);
+    for (int s = 0; s < C::WS; ++s) mbar_init(smem_u32(&aux->wfull[s]), 1 + 32);   // the producer and the scale warp's lanes
+    for (int s = 0; s < C::PS; ++s) {
+      mbar_init(smem_u32(&aux->pfull[s]), 1);
+      mbar_init(smem_u32(&aux->pdone[s]), 1);
     }
     for (int b = 0; b < C::NBUF; ++b) mbar_init(smem_u32(&aux->tempty[b]), kLEpiWarps);
     mbar_init(smem_u32(&aux->esync), kLEpiThreads);
     fence_mbar_init();
     tma_prefetch_desc(&tm_w);
-    tma_prefetch_desc(&tm_b);
+    for (int i = 0; i < 4; ++i) tma_prefetch_desc(&tm_b.m[i]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&aux->tmem_base), C::TMEM_COLS);
@@ -157,77 +194,125 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   tc_fence_after_sync();
   const uint32_t tmem_base = aux->tmem_base;
   volatile int* abort_flag = &aux->abort;
+  const uint32_t smem_base = smem_u32(smem), tok_base = smem_base + C::WS * C::W_BYTES;
+  const uint32_t wfull_base = smem_u32(&aux->wfull[0]), pfull_base = smem_u32(&aux->pfull[0]);
+  const uint32_t pdone_base = smem_u32(&aux->pdone[0]), tempty_base = smem_u32(&aux->tempty[0]);
+  constexpr bool JOINT = C::NTERMS == 1;      // tokens and weights of a K-block on one barrier
 
   if (warp < kLFirstEpi) {
     setmaxnreg_dec<kLRegsControl>();
+    bool ok = true;
+    Pos<C::WS> wp;
+    Pos<C::PS> pp, old;        // next plane; last plane of the K-block that used the weight slot before
+    old.step(C::NTERMS - 1);
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
-        const uint32_t smem_base = smem_u32(smem);
-        const uint32_t full_base = smem_u32(&aux->full[0]), done_base = smem_u32(&aux->done[0]);
-        uint32_t stage = 0, ph = 0;
-        bool ok = true;
-        for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
-          const LItem w = decode_large<GEMM>(i, aux);
+      int n = 0;
+      for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
+        const LItem w = decode_large<GEMM>(i, aux);
+        const int steps = (w.valid + kRowStep - 1) / kRowStep;      // a ragged tile brings the rows it has
+        const CUtensorMap* mb = &tm_b.m[steps - 1];
+        const uint32_t tok_tx = static_cast<uint32_t>(steps) * (kRowStep * 128);
 #pragma unroll 1
-          for (int kb = 0; kb < C::KB; ++kb) {
-            if (!mbar_wait(done_base + stage * 8, ph ^ 1u, abort_flag)) { ok = false; break; }
-            const uint32_t bar = full_base + stage * 8;
-            mbar_arrive_expect_tx(bar, C::STAGE_BYTES);
-            const uint32_t dst = smem_base + stage * C::STAGE_BYTES;
+        for (int kb = 0; kb < C::KB; ++kb, ++n, wp.step()) {
+          if (n >= C::WS) {
+            if (!mbar_wait(pdone_base + old.i * 8, old.ph, abort_flag)) { ok = false; break; }
+            old.step(C::NTERMS);
+          }
+          if (elect_one()) {
+            const uint32_t bar = wfull_base + wp.i * 8;
+            const uint32_t dst = smem_base + wp.i * C::W_BYTES;
+            mbar_arrive_expect_tx(bar, C::W_BYTES + (JOINT ? tok_tx : 0u));
             if constexpr (GEMM == 1) {
               // weights: 128 rows of the first half of W13 | the same 128 rows of the second half
               const int y = w.e * k2I + w.j * 128;
               tma_load_3d(dst, &tm_w, 0, y, kb, bar);
               tma_load_3d(dst + 128 * 128, &tm_w, 0, y + kI, kb, bar);
-              tma_load_3d(dst + C::W_BYTES, &tm_b, 0, w.row0, kb, bar);                   // [128 rows][128 B]
+              tma_load_3d(tok_base + pp.i * C::TOK_BYTES, mb, 0, w.row0, kb, bar);
             } else {
               tma_load_3d(dst, &tm_w, 0, w.e * kH + w.j * 256, kb, bar);                  // 256 weight rows as two boxes
               tma_load_3d(dst + 128 * 128, &tm_w, 0, w.e * kH + w.j * 256 + 128, kb, bar);
-              tma_load_4d(dst + C::W_BYTES, &tm_b, 0, w.row0, 0, kb, bar);                // [3 planes][128 rows][128 B]
             }
-            if (++stage == C::STAGES) { stage = 0; ph ^= 1u; }
+          }
+          if constexpr (JOINT) {
+            pp.step();
+          } else {
+            for (int t = 0; t < C::NTERMS; ++t, pp.step()) {
+              if (!mbar_wait(pdone_base + pp.i * 8, pp.ph ^ 1u, abort_flag)) { ok = false; break; }
+              if (elect_one()) {
+                const uint32_t bar = pfull_base + pp.i * 8;
+                mbar_arrive_expect_tx(bar, tok_tx);
+                tma_load_4d(tok_base + pp.i * C::TOK_BYTES, mb, 0, w.row0, t, kb, bar);
+              }
+            }
+            if (!ok) break;
           }
         }
       }
-      __syncwarp();   // block-wide barriers below need whole warps
-    } else if (warp == 1 || warp == 2) {
-      // ------------------------------------------------------------------ UMMA issuers (alternate stages)
-      if (lane == 0) {
-        constexpr uint32_t idesc = umma_idesc_e4m3(128, C::W_ROWS);
-        const uint64_t desc_const = umma_desc_k_sw128(0);
-        const uint32_t smem_base = smem_u32(smem);
-        const uint32_t full_base = smem_u32(&aux->full[0]), done_base = smem_u32(&aux->done[0]);
-        const uint32_t tempty_base = smem_u32(&aux->tempty[0]);
-        uint32_t stage = 0, ph = 0, buf = 0, bph = 0;
-        bool ok = true;
-        int nst = 0;
-        for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
+    } else if (warp == 3) {
+      // ------------------------------------------------------------------ scales of every K-block
+      uint32_t slot = smem_u32(slots);
+      const uint32_t slot_end = slot + C::NSLOT * C::SLOT_FLOATS * 4;
+      int n = 0;
+      for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
+        const LItem w = decode_large<GEMM>(i, aux);
+        // the two 128-row weight blocks of the item: GEMM1 j and j + 16, GEMM2 2 j and 2 j + 1
+        const float* wsp = a.w_scale + (GEMM == 1 ? (static_cast<size_t>(w.e) * kMT1 + w.j + (lane & 1) * kKB2) * kKB1
+                                                  : (static_cast<size_t>(w.e) * kMT2 + 2 * w.j + (lane & 1)) * kKB2);
 #pragma unroll 1
-          for (int s = 0; s < C::KB; ++s, ++nst) {
-            if ((nst & 1) == warp - 1) {
-              if (!mbar_wait(tempty_base + buf * 8, bph ^ 1u, abort_flag)) { ok = false; break; }
-              if (!mbar_wait(full_base + stage * 8, ph, abort_flag)) { ok = false; break; }
-              tc_fence_after_sync();
-              const uint32_t sbase = smem_base + stage * C::STAGE_BYTES;
-              const uint64_t wdesc = desc_const | (sbase >> 4);
-              const uint32_t d = tmem_base + buf * C::BUF_COLS;
+        for (int kb = 0; kb < C::KB; ++kb, ++n, wp.step()) {
+          if (n >= C::WS) {
+            if (!mbar_wait(pdone_base + old.i * 8, old.ph, abort_flag)) { ok = false; break; }
+            old.step(C::NTERMS);
+          }
+          const float* bsp = a.b_scale + static_cast<size_t>(kb) * a.rows_cap;
 #pragma unroll
-              for (int t = 0; t < C::NTERMS; ++t) {
-                const uint64_t tdesc = desc_const | ((sbase + C::W_BYTES + t * C::TOK_BYTES) >> 4);
+          for (int j0 = 0; j0 < 128; j0 += 32)    // rows past the tile's last one: any value, they are dropped
+            if (j0 < w.valid) cp_async4(slot + (j0 + lane) * 4, bsp + min(w.row0 + j0 + lane, a.rows_cap - 1));
+          if (lane < 2) cp_async4(slot + (128 + lane) * 4, wsp + kb);
+          cp_async_arrive(wfull_base + wp.i * 8);
+          slot += C::SLOT_FLOATS * 4;
+          if (slot == slot_end) slot = smem_u32(slots);
+        }
+      }
+    } else {
+      // ------------------------------------------------------------------ UMMA issuers (alternate K-blocks)
+      constexpr uint32_t idesc = umma_idesc_e4m3(128, C::W_ROWS);
+      const uint64_t desc_const = umma_desc_k_sw128(0);
+      Pos<C::NBUF> tb;
+      int n = 0;
+      for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
+#pragma unroll 1
+        for (int s = 0; s < C::KB; ++s, ++n) {
+          if ((n & 1) == warp - 1) {
+            if (!mbar_wait(tempty_base + tb.i * 8, tb.ph ^ 1u, abort_flag)) { ok = false; break; }
+            if (!mbar_wait(wfull_base + wp.i * 8, wp.ph, abort_flag)) { ok = false; break; }
+            const uint64_t wdesc = desc_const | ((smem_base + wp.i * C::W_BYTES) >> 4);
+            const uint32_t d = tmem_base + tb.i * C::BUF_COLS;
+#pragma unroll
+            for (int t = 0; t < C::NTERMS; ++t, pp.step()) {
+              if constexpr (!JOINT) {
+                if (!mbar_wait(pfull_base + pp.i * 8, pp.ph, abort_flag)) { ok = false; break; }
+              }
+              tc_fence_after_sync();
+              if (elect_one()) {
+                const uint64_t tdesc = desc_const | ((tok_base + pp.i * C::TOK_BYTES) >> 4);
 #pragma unroll
                 for (int k4 = 0; k4 < 4; ++k4)   // +32 bytes of K inside the 128-byte swizzle atom = +2 encoded units
                   umma_f8(d, tdesc + 2 * k4, wdesc + 2 * k4, idesc, (t | k4) != 0 ? 1u : 0u);
+                umma_commit(pdone_base + pp.i * 8);
               }
-              umma_commit(done_base + stage * 8);
             }
-            if (++stage == C::STAGES) { stage = 0; ph ^= 1u; }
-            if (++buf == C::NBUF) { buf = 0; bph ^= 1u; }
+            if (!ok) break;
+          } else {
+            pp.step(C::NTERMS);
           }
+          wp.step();
+          tb.step();
         }
       }
-      __syncwarp();
     }
+    __syncwarp();   // block-wide barriers below need whole warps
   } else {
     setmaxnreg_inc<kLRegsEpi>();
     // ------------------------------------------------------------------ promotion + epilogue (warps 4..19)
@@ -235,8 +320,15 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     const int cg = (warp - kLFirstEpi) >> 2;      // column group: a quarter of the accumulator columns
     const int trow = q * 32 + lane;               // token row inside the tile
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    const uint32_t done_base = smem_u32(&aux->done[0]), tempty_base = smem_u32(&aux->tempty[0]);
-    uint32_t stage = 0, ph = 0, buf = 0, bph = 0;      // same ring positions as the issuers
+    Pos<C::PS> last;                              // last plane of the next K-block
+    last.step(C::NTERMS - 1);
+    Pos<C::NBUF> tb;
+    int slot = 0;
+    auto release = [&]() {
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty_base + tb.i * 8);
+    };
     uint32_t eph = 0;
     bool ok = true;
     auto epi_sync = [&]() {
@@ -247,38 +339,33 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
       const LItem w = decode_large<GEMM>(i, aux);
       const int row = w.row0 + trow;
-      const int lrow = min(row, a.rows_cap - 1);   // rows past the tile's last one are computed and dropped
-      if constexpr (GEMM == 1) {
-        // scales of this thread's token row and of the item's two weight blocks, read one K-block ahead
-        const float* bsp = a.b_scale + lrow;   // [56][rows_cap]: a warp's 32 rows are one line
-        const float* w1p = a.w_scale + (static_cast<size_t>(w.e) * kMT1 + w.j) * kKB1;
-        const float* w2p = w1p + kKB2 * kKB1;   // the block 16 further: the second half of W13
-        float acc[64];      // [0, 32): x1 of this thread's 32 columns, [32, 64): x2 of the same columns
+      float acc[64];      // GEMM1: [0, 32) x1 of this thread's 32 columns, [32, 64) x2 of the same; GEMM2: 64 columns
 #pragma unroll
-        for (int x = 0; x < 64; ++x) acc[x] = 0.0f;
-        float nb = __ldg(bsp), n1 = __ldg(w1p), n2 = __ldg(w2p);
+      for (int x = 0; x < 64; ++x) acc[x] = 0.0f;
+      const bool live = q * 32 < w.valid;         // a warp whose rows lie past the tile's last one reads nothing
 #pragma unroll 1
-        for (int s = 0; s < kKB1; ++s) {
-          if (!mbar_wait(done_base + stage * 8, ph, abort_flag)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t taddr = tmem_base + lane_addr + buf * C::BUF_COLS + cg * 32;
-          float v[32];
-          tmem_ld32(taddr, v);                  // x1: columns cg*32 .. +32 of the first 128
-          // (scale arithmetic and the next K-block's scale loads run under the read-back's latency)
-          const float f1 = n1 * nb, f2 = n2 * nb;
-          if (s + 1 < kKB1) { nb = __ldg(bsp + static_cast<size_t>(s + 1) * a.rows_cap); n1 = __ldg(w1p + s + 1); n2 = __ldg(w2p + s + 1); }
-          tmem_wait_ld();
-          fma_scaled<32>(acc, v, f1);
-          tmem_ld32(taddr + 128, v);            // x2: the same columns of the second 128
-          tmem_wait_ld();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(tempty_base + buf * 8);
-          fma_scaled<32>(acc + 32, v, f2);
-          if (++stage == C::STAGES) { stage = 0; ph ^= 1u; }
-          if (++buf == C::NBUF) { buf = 0; bph ^= 1u; }
-        }
-        if (!ok) break;
+      for (int s = 0; s < C::KB; ++s, last.step(C::NTERMS), tb.step()) {
+        if (!mbar_wait(pdone_base + last.i * 8, last.ph, abort_flag)) { ok = false; break; }
+        tc_fence_after_sync();
+        const float* sl = slots + slot * C::SLOT_FLOATS;
+        if (++slot == C::NSLOT) slot = 0;
+        if (!live) { release(); continue; }
+        const uint32_t taddr = tmem_base + lane_addr + tb.i * C::BUF_COLS + cg * (GEMM == 1 ? 32 : 64);
+        float v[32];
+        tmem_ld32(taddr, v);
+        // GEMM1: the halves belong to two weight blocks; GEMM2: this thread's 64 columns lie in one, 2 j + (cg >> 1)
+        const float nb = sl[trow];
+        const float f1 = sl[128 + (GEMM == 1 ? 0 : cg >> 1)] * nb;
+        const float f2 = GEMM == 1 ? sl[129] * nb : f1;
+        tmem_wait_ld();
+        fma_scaled<32>(acc, v, f1);
+        tmem_ld32(taddr + (GEMM == 1 ? 128 : 32), v);
+        tmem_wait_ld();
+        release();
+        fma_scaled<32>(acc + 32, v, f2);
+      }
+      if (!ok) break;
+      if constexpr (GEMM == 1) {
         float amax = 0.0f;
 #pragma unroll
         for (int x = 0; x < 32; ++x) {
@@ -316,35 +403,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
           }
         }
       } else {
-        // this thread's 64 columns lie in ONE 128-row weight block: 2 j + (cg >> 1)
-        const int tile = 2 * w.j + (cg >> 1);
-        const float* bsp = a.b_scale + lrow;   // [16][rows_cap]
-        const float* wsp = a.w_scale + (static_cast<size_t>(w.e) * kMT2 + tile) * kKB2;
-        float acc[64];
-#pragma unroll
-        for (int x = 0; x < 64; ++x) acc[x] = 0.0f;
-        float nb = __ldg(bsp), nw = __ldg(wsp);
-#pragma unroll 1
-        for (int s = 0; s < kKB2; ++s) {
-          if (!mbar_wait(done_base + stage * 8, ph, abort_flag)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t taddr = tmem_base + lane_addr + buf * C::BUF_COLS + cg * 64;
-          float v[32];
-          tmem_ld32(taddr, v);
-          const float f = nw * nb;
-          if (s + 1 < kKB2) { nb = __ldg(bsp + static_cast<size_t>(s + 1) * a.rows_cap); nw = __ldg(wsp + s + 1); }
-          tmem_wait_ld();
-          fma_scaled<32>(acc, v, f);
-          tmem_ld32(taddr + 32, v);
-          tmem_wait_ld();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(tempty_base + buf * 8);
-          fma_scaled<32>(acc + 32, v, f);
-          if (++stage == C::STAGES) { stage = 0; ph ^= 1u; }
-          if (++buf == C::NBUF) { buf = 0; bph ^= 1u; }
-        }
-        if (!ok) break;
+        const int tile = 2 * w.j + (cg >> 1);     // the 128-row weight block of this thread's columns
         if (trow < w.valid) {
           const int col0 = w.j * 256 + cg * 64;
           if constexpr (!COMBINE) {
@@ -432,7 +491,7 @@ int grouped_gemm_large_init() {
   return 0;
 }
 
-int launch_grouped_gemm_large(int gemm_id, bool fused_combine, const CUtensorMap& tm_w, const CUtensorMap& tm_b,
+int launch_grouped_gemm_large(int gemm_id, bool fused_combine, const CUtensorMap& tm_w, const TokenMaps& tm_b,
                               const GemmArgs& a, int ctas, cudaStream_t stream) {
   if (gemm_id == 1)
     return static_cast<int>(launch_pdl(grouped_gemm_large_kernel<1, false>, dim3(ctas), dim3(kLThreads),

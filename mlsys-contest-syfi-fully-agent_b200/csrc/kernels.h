@@ -133,13 +133,13 @@ void launch_route_permute(const RouteArgs& r, const PermuteArgs& p, cudaStream_t
 void launch_route_only(const RouteArgs& r, cudaStream_t stream);
 void launch_gather_rows(const GatherArgs& a, int T, cudaStream_t stream);
 // gemm_id 1 or 2; n_tile in {32, 64, 128}.  Returns a cudaError_t as int.
-// Token-operand tensor maps of grouped_gemm_kernel: the same tensor with boxes of 1..4 row steps
-// (32 rows each), so that a token tile with few valid rows (the last tile of an
+// Token-operand tensor maps of the grouped GEMM kernels: the same tensor with boxes of 1..4 row steps, so that a token tile with few valid rows (the last tile of an
 // expert, or an expert with a handful of tokens) brings only the rows it has, rounded up to a step.
 struct TokenMaps {
   CUtensorMap m[4];
 };
 int grouped_gemm_row_step(int n_tile);
+constexpr int kLargeRowStep = 32;   // row step of the large-batch kernels (one TMEM lane quarter)
 int launch_grouped_gemm(int gemm_id, int n_tile, const CUtensorMap& tm_w, const TokenMaps& tm_b, const GemmArgs& a,
                         int ctas, cudaStream_t stream);
 constexpr int kFusedMaxTokens = 16;
@@ -154,7 +154,7 @@ int grouped_gemm_init();   // one-time function attributes (dynamic shared memor
 // Large batches (128-token tiles): GEMM1 with SwiGLU and the e4m3 plane split in its epilogue; GEMM2 storing fp32 rows
 // for the deterministic combine kernel, or (fused_combine) adding weighted rows into acc32 with a last-arriver bf16 cast.
 int grouped_gemm_large_init();
-int launch_grouped_gemm_large(int gemm_id, bool fused_combine, const CUtensorMap& tm_w, const CUtensorMap& tm_b,
+int launch_grouped_gemm_large(int gemm_id, bool fused_combine, const CUtensorMap& tm_w, const TokenMaps& tm_b,
                               const GemmArgs& a, int ctas, cudaStream_t stream);
 // Zeroes `acc_floats` floats at acc32 (the accumulator and the counters behind it) and writes zero output rows for
 // tokens without a local expert.

@@ -180,14 +180,14 @@ MapKey kblock_map(const void* ptr, uint64_t rows, uint64_t K, uint32_t box_rows,
 }
 
 // The kNTerms e4m3 planes [plane][rows, 2048] of GEMM2's token operand as
-// [128 B, rows, planes, K-blocks]: one box brings all planes of `kps` K-blocks, plane-major inside a K-block.
-MapKey planes_map(const void* ptr, uint64_t rows, uint32_t box_rows, uint32_t kps) {
+// [128 B, rows, planes, K-blocks]: one box brings `box_planes` planes of `kps` K-blocks, plane-major inside a K-block.
+MapKey planes_map(const void* ptr, uint64_t rows, uint32_t box_rows, uint32_t kps, uint32_t box_planes = kNTerms) {
   MapKey k{};
   k.ptr = ptr;
   k.rank = 4;
   k.dims[0] = 128; k.dims[1] = rows; k.dims[2] = kNTerms; k.dims[3] = kI / 128;
   k.strides[0] = kI; k.strides[1] = rows * kI; k.strides[2] = 128;
-  k.box[0] = 128; k.box[1] = box_rows; k.box[2] = kNTerms; k.box[3] = kps;
+  k.box[0] = 128; k.box[1] = box_rows; k.box[2] = box_planes; k.box[3] = kps;
   return k;
 }
 
@@ -302,7 +302,7 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
   const int n_tile2 = (T > 32 && T <= 768) ? 32 : n_tile > 128 ? 128 : n_tile;
   const int ctas = dev->sm_count;
 
-  CUtensorMap tm_w13, tm_w2, tm_a, tm_c;
+  CUtensorMap tm_w13, tm_w2;
   const bool decode = T <= kFusedMaxTokens;
   const uint32_t kps1 = decode ? kDecodeKps : grouped_gemm_kblocks_per_stage(1, n_tile);
   const uint32_t kps2 = decode ? kDecodeKps : grouped_gemm_kblocks_per_stage(2, n_tile2);
@@ -311,15 +311,14 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
     return rc;
   if ((rc = get_map(dev, kblock_map(gemm2_weights, static_cast<uint64_t>(kELocal) * kH, kI, 128, kps2), &tm_w2)))
     return rc;
-  if ((rc = get_map(dev, kblock_map(a_packed, L.rows_cap, kH, n_tile, large ? 1 : kps1), &tm_a))) return rc;
-  if ((rc = get_map(dev, planes_map(cq, L.rows_cap, n_tile2, kps2), &tm_c))) return rc;
 
   if (T <= kFusedMaxTokens) {
     // Decode path: one launch.  The kernel routes, reads the token rows straight from hidden_states (all
     // tokens are one token tile), and runs both GEMMs with the SwiGLU and combine phases in between and after.
-    CUtensorMap tm_h;
+    CUtensorMap tm_h, tm_c;
     if ((rc = get_map(dev, kblock_map(hidden_states, static_cast<uint64_t>(T), kH, kFusedMaxTokens, kps1), &tm_h)))
       return rc;
+    if ((rc = get_map(dev, planes_map(cq, L.rows_cap, n_tile2, kps2), &tm_c))) return rc;
     GemmArgs fa{};
     fa.sched = sched; fa.w_scale = gemm1_weights_scale; fa.b_scale = nullptr; fa.out = g1;
     fa.logits = routing_logits; fa.bias_bf16 = routing_bias; fa.hidden_scale = hidden_states_scale;
@@ -362,6 +361,17 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
   g2a.rows_cap = L.rows_cap; g2a.perm_token = perm_token; g2a.perm_weight = perm_weight; g2a.local_mask = local_mask;
   g2a.acc32 = acc32; g2a.tile_cnt = tile_cnt; g2a.out_bf16 = output; g2a.out_rows = output_rows;
 
+  // token operands with boxes of 1..4 row steps (ragged token tiles bring only the rows they have)
+  TokenMaps tms_a, tms_c;
+  const int step1 = large ? kLargeRowStep : grouped_gemm_row_step(n_tile);
+  const int step2 = large ? kLargeRowStep : grouped_gemm_row_step(n_tile2);
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t r1 = static_cast<uint32_t>(std::min(n_tile, step1 * (i + 1)));
+    const uint32_t r2 = static_cast<uint32_t>(std::min(n_tile2, step2 * (i + 1)));
+    if ((rc = get_map(dev, kblock_map(a_packed, L.rows_cap, kH, r1, large ? 1 : kps1), &tms_a.m[i]))) return rc;
+    if ((rc = get_map(dev, planes_map(cq, L.rows_cap, r2, kps2, large ? 1 : kNTerms), &tms_c.m[i]))) return rc;
+  }
+
   if (large) {
     if (fast_combine) {
       // accumulator + counters are one span of the workspace
@@ -372,29 +382,20 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
       }
       g_launches += 1;
     }
-    if ((rc = launch_grouped_gemm_large(1, false, tm_w13, tm_a, g1a, ctas, stream))) {
+    if ((rc = launch_grouped_gemm_large(1, false, tm_w13, tms_a, g1a, ctas, stream))) {
       g_last_cuda_error = rc;
       return MOE_B200_ECUDA;
     }
     g_launches += 1;
     stage_mark(3, stream);
     stage_mark(4, stream);      // no SwiGLU kernel on this path
-    if ((rc = launch_grouped_gemm_large(2, fast_combine, tm_w2, tm_c, g2a, ctas, stream))) {
+    if ((rc = launch_grouped_gemm_large(2, fast_combine, tm_w2, tms_c, g2a, ctas, stream))) {
       g_last_cuda_error = rc;
       return MOE_B200_ECUDA;
     }
     g_launches += 1;
     stage_mark(5, stream);
   } else {
-    // token operands with boxes of 1..4 row steps (ragged token tiles bring only the rows they have)
-    TokenMaps tms_a, tms_c;
-    const int step1 = grouped_gemm_row_step(n_tile), step2 = grouped_gemm_row_step(n_tile2);
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t r1 = static_cast<uint32_t>(std::min(n_tile, step1 * (i + 1)));
-      const uint32_t r2 = static_cast<uint32_t>(std::min(n_tile2, step2 * (i + 1)));
-      if ((rc = get_map(dev, kblock_map(a_packed, L.rows_cap, kH, r1, kps1), &tms_a.m[i]))) return rc;
-      if ((rc = get_map(dev, planes_map(cq, L.rows_cap, r2, kps2), &tms_c.m[i]))) return rc;
-    }
     if ((rc = launch_grouped_gemm(1, n_tile, tm_w13, tms_a, g1a, ctas, stream))) {
       g_last_cuda_error = rc;
       return MOE_B200_ECUDA;
