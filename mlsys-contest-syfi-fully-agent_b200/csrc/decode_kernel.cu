@@ -14,8 +14,8 @@
 // the second grid barrier.  A stage's "full" barrier expects the bytes of both boxes, so the UMMA issuer
 // needs no knowledge of the split.
 //
-//   warp 0      TMA producer (one thread)          warps 4-11  promotion + epilogue + tails
-//   warp 1      UMMA issuer  (one thread)          (same roles and ring protocol as grouped_gemm.cu)
+//   warp 0      TMA producer (elected lane)        warps 4-11  promotion + epilogue + tails
+//   warp 1      UMMA issuer  (elected lane)        (same roles and ring protocol as grouped_gemm.cu)
 //
 // Work split ("stream-K"): a GEMM's work is the sequence of pipeline stages (2 K-blocks) of all its
 // (expert, weight-row tile) pairs, tile-major; CTA c takes the stages [c*G/n, (c+1)*G/n), i.e. a contiguous
@@ -123,7 +123,7 @@ struct Ring {
   }
 };
 
-// UMMA issue of one GEMM's items (one thread).
+// UMMA issue of one GEMM's items (a whole warp; one elected lane issues).
 template <int GEMM>
 __device__ __forceinline__ bool issue_items(int tiles, const Aux* aux, uint32_t smem_base, uint32_t tmem_base, Ring& r,
                                             volatile int* abort_flag) {
@@ -142,16 +142,18 @@ __device__ __forceinline__ bool issue_items(int tiles, const Aux* aux, uint32_t 
       if (!mbar_wait(tempty_base + r.buf * 8, r.bph ^ 1u, abort_flag)) return false;
       if (!mbar_wait(full_base + r.stage * 8, r.ph, abort_flag)) return false;
       tc_fence_after_sync();
-      const uint32_t sbase = smem_base + r.stage * DC::STAGE_BYTES;
+      if (elect_one()) {
+        const uint32_t sbase = smem_base + r.stage * DC::STAGE_BYTES;
 #pragma unroll
-      for (int u = 0; u < DC::KPS; ++u) {
-        const uint64_t adesc = desc_const | ((sbase + u * DC::A_BYTES) >> 4);
-        const uint64_t bdesc = desc_const | ((sbase + DC::B_OFF + u * BB) >> 4);
-        const uint32_t d = tmem_base + r.buf * DC::BUF_COLS + u * COLS;
+        for (int u = 0; u < DC::KPS; ++u) {
+          const uint64_t adesc = desc_const | ((sbase + u * DC::A_BYTES) >> 4);
+          const uint64_t bdesc = desc_const | ((sbase + DC::B_OFF + u * BB) >> 4);
+          const uint32_t d = tmem_base + r.buf * DC::BUF_COLS + u * COLS;
 #pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) umma_f8(d, adesc + 2 * k4, bdesc + 2 * k4, idesc, k4 != 0 ? 1u : 0u);
+          for (int k4 = 0; k4 < 4; ++k4) umma_f8(d, adesc + 2 * k4, bdesc + 2 * k4, idesc, k4 != 0 ? 1u : 0u);
+        }
+        umma_commit(done_base + r.stage * 8);
       }
-      umma_commit(done_base + r.stage * 8);
       r.advance();
     }
   }
@@ -321,7 +323,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
   Aux* aux = reinterpret_cast<Aux*>(smem + DC::STAGES * DC::STAGE_BYTES + DC::SC_BYTES);
   FusedAux* fa = reinterpret_cast<FusedAux*>(reinterpret_cast<uint8_t*>(aux) + 1024);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   griddep_launch_dependents();
   MoeSched* sched = a.g.sched;
@@ -369,7 +371,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
     setmaxnreg_dec<kRegsControl>();
     if (warp == 0) {
       // ---------------------------------------------------------------- TMA producer
-      if (lane == 0) {
+      {
         const uint32_t smem_base = smem_u32(smem);
         const uint32_t full_base = smem_u32(&aux->full[0]), done_base = smem_u32(&aux->done[0]);
         uint32_t stage = 0, ph = 0;
@@ -382,11 +384,13 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
             const int wy = w.e * k2I + w.m * 128;
             for (int kb = w.kb0; kb < w.kb1; kb += DC::KPS) {
               if (!mbar_wait(done_base + stage * 8, ph ^ 1u, abort_flag)) { ok = false; break; }
-              const uint32_t fb = full_base + stage * 8;
-              mbar_arrive_expect_tx(fb, DC::TX1);
-              const uint32_t dst = smem_base + stage * DC::STAGE_BYTES;
-              tma_load_3d(dst, &tm_w1, 0, wy, kb, fb);                 // [2 K-blocks][128 rows][128 B]
-              tma_load_3d(dst + DC::B_OFF, &tm_x, 0, 0, kb, fb);       // [2 K-blocks][16 tokens][128 B]
+              if (elect_one()) {
+                const uint32_t fb = full_base + stage * 8;
+                mbar_arrive_expect_tx(fb, DC::TX1);
+                const uint32_t dst = smem_base + stage * DC::STAGE_BYTES;
+                tma_load_3d(dst, &tm_w1, 0, wy, kb, fb);                 // [2 K-blocks][128 rows][128 B]
+                tma_load_3d(dst + DC::B_OFF, &tm_x, 0, 0, kb, fb);       // [2 K-blocks][16 tokens][128 B]
+              }
               if (++stage == DC::STAGES) { stage = 0; ph ^= 1u; }
             }
           }
@@ -413,7 +417,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
                 bool phave = whave;
                 int pkb = wkb;
                 for (int n = 0; phave && n < kL2PrefetchStages; ++n) {
-                  tma_prefetch_l2_3d(&tm_w2, 0, pw.e * kH + pw.m * 128, pkb);
+                  if (elect_one()) tma_prefetch_l2_3d(&tm_w2, 0, pw.e * kH + pw.m * 128, pkb);
                   pkb += DC::KPS;
                   if (pkb >= pw.kb1) {
                     phave = ppart.next(aux, pw);
@@ -425,8 +429,9 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
               fence_proxy_async_global();   // the planes were written with ordinary stores by other SMs
               ready = true;
             }
-            tma_load_4d(smem_base + bstage * DC::STAGE_BYTES + DC::B_OFF, &tm_c, 0, bw.row0, 0, bkb,
-                        full_base + bstage * 8);                     // [2 K-blocks][3 planes][16 rows][128 B]
+            if (elect_one())
+              tma_load_4d(smem_base + bstage * DC::STAGE_BYTES + DC::B_OFF, &tm_c, 0, bw.row0, 0, bkb,
+                          full_base + bstage * 8);                   // [2 K-blocks][3 planes][16 rows][128 B]
             if (++bstage == DC::STAGES) bstage = 0;
             --ahead;
             bkb += DC::KPS;
@@ -436,9 +441,11 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
             }
           } else {
             if (!mbar_wait(done_base + stage * 8, ph ^ 1u, abort_flag)) { ok = false; break; }
-            const uint32_t fb = full_base + stage * 8;
-            mbar_arrive_expect_tx(fb, DC::TX2);
-            tma_load_3d(smem_base + stage * DC::STAGE_BYTES, &tm_w2, 0, ww.e * kH + ww.m * 128, wkb, fb);
+            if (elect_one()) {
+              const uint32_t fb = full_base + stage * 8;
+              mbar_arrive_expect_tx(fb, DC::TX2);
+              tma_load_3d(smem_base + stage * DC::STAGE_BYTES, &tm_w2, 0, ww.e * kH + ww.m * 128, wkb, fb);
+            }
             if (++stage == DC::STAGES) { stage = 0; ph ^= 1u; }
             ++ahead;
             wkb += DC::KPS;
@@ -452,12 +459,10 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
       __syncwarp();   // block-wide barriers below need whole warps
     } else if (warp == 1) {
       // ---------------------------------------------------------------- UMMA issuer
-      if (lane == 0) {
-        Ring r;
-        const uint32_t smem_base = smem_u32(smem);
-        if (issue_items<1>(tiles, aux, smem_base, tmem_base, r, abort_flag))
-          issue_items<2>(tiles, aux, smem_base, tmem_base, r, abort_flag);
-      }
+      Ring r;
+      const uint32_t smem_base = smem_u32(smem);
+      if (issue_items<1>(tiles, aux, smem_base, tmem_base, r, abort_flag))
+        issue_items<2>(tiles, aux, smem_base, tmem_base, r, abort_flag);
       __syncwarp();
     }
   } else {
