@@ -238,6 +238,35 @@ def test_fused_large_batch_path_against_unfused_path(pkg, dev, W, options, T, se
     assert m["cosine"] >= 0.999999 and m["match_ratio"] == 1.0
 
 
+@pytest.mark.parametrize("counts", [[1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160], [255, 256, 257, 1]])
+def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, options, counts):
+    """Experts whose row counts sit at the edges of the 32-row steps and of the 128-token tiles: every token with work
+    selects exactly one local expert, `counts[e]` tokens expert e, and the batch is filled up with tokens that have
+    none.  The planes carry the same fp32 operations in the same order on both paths: equal bit for bit."""
+    T = max(1100, sum(counts) + 5)
+    tok = pkg.gen.make_tokens(T, 11, dev)
+    logits = tok.routing_logits * 0.01 - 6.0
+    logits[:, 32:35] += 12.0                      # seven experts of groups 1 to 3 for everybody
+    logits[:, 64:66] += 12.0
+    logits[:, 96:98] += 12.0
+    logits[:, 130] += 6.0                         # the eighth, where no local expert scores higher
+    expert = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    logits[torch.arange(len(expert), device=dev), expert.to(dev)] += 12.0
+    tok.routing_logits = logits.contiguous()
+    tok.routing_bias = torch.zeros_like(tok.routing_bias)
+    options(pkg.loader.OPT_UNFUSED)
+    out_u = run_op(pkg, tok, W, 0).clone()
+    cq_u, cs_u = ws_readers.swiglu_planes(pkg, T)
+    options(0)
+    out_f = run_op(pkg, tok, W, 0).clone()
+    cq_f, cs_f = ws_readers.swiglu_planes(pkg, T)
+    assert cq_u.shape[1] == sum(counts)
+    assert torch.equal(cs_u, cs_f) and torch.equal(cq_u, cq_f)
+    assert float(out_f[sum(counts):].float().abs().max()) == 0.0
+    m = moe_oracle.output_metrics(out_f, out_u, out_u.float())
+    assert m["cosine"] >= 0.999999 and m["match_ratio"] == 1.0
+
+
 @pytest.mark.parametrize("T,seed,skew,offset", [(4096, 0, False, 0), (1100, 3, True, 0), (6000, 5, False, 96)])
 def test_fast_combine_against_oracle(pkg, dev, W, options, T, seed, skew, offset):
     """MOE_B200_OPT_FAST_COMBINE: routing-weight multiply and fp32 combine in GEMM2's epilogue (vector reductions,
