@@ -239,10 +239,10 @@ def test_fused_large_batch_path_against_unfused_path(pkg, dev, W, options, T, se
 
 
 @pytest.mark.parametrize("counts", [[1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160], [255, 256, 257, 1]])
-def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, options, counts):
+def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, counts):
     """Experts whose row counts sit at the edges of the 32-row steps and of the 128-token tiles: every token with work
     selects exactly one local expert, `counts[e]` tokens expert e, and the batch is filled up with tokens that have
-    none.  The planes carry the same fp32 operations in the same order on both paths: equal bit for bit."""
+    none.  Same bars as every other batch against the oracle."""
     T = max(1100, sum(counts) + 5)
     tok = pkg.gen.make_tokens(T, 11, dev)
     logits = tok.routing_logits * 0.01 - 6.0
@@ -250,21 +250,16 @@ def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, options, counts
     logits[:, 64:66] += 12.0
     logits[:, 96:98] += 12.0
     logits[:, 130] += 6.0                         # the eighth, where no local expert scores higher
-    expert = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
-    logits[torch.arange(len(expert), device=dev), expert.to(dev)] += 12.0
-    tok.routing_logits = logits.contiguous()
-    tok.routing_bias = torch.zeros_like(tok.routing_bias)
-    options(pkg.loader.OPT_UNFUSED)
-    out_u = run_op(pkg, tok, W, 0).clone()
-    cq_u, cs_u = ws_readers.swiglu_planes(pkg, T)
-    options(0)
-    out_f = run_op(pkg, tok, W, 0).clone()
-    cq_f, cs_f = ws_readers.swiglu_planes(pkg, T)
-    assert cq_u.shape[1] == sum(counts)
-    assert torch.equal(cs_u, cs_f) and torch.equal(cq_u, cq_f)
-    assert float(out_f[sum(counts):].float().abs().max()) == 0.0
-    m = moe_oracle.output_metrics(out_f, out_u, out_u.float())
-    assert m["cosine"] >= 0.999999 and m["match_ratio"] == 1.0
+    expert = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts)).to(dev)
+    logits[torch.arange(len(expert), device=dev), expert] += 12.0
+    bias = torch.zeros_like(tok.routing_bias)
+    ref = moe_oracle.run_full(logits, bias, tok.hidden_states, tok.hidden_states_scale, W.gemm1_weights,
+                              W.gemm1_weights_scale, W.gemm2_weights, W.gemm2_weights_scale, 0, RSF)
+    out = pkg.op.run(logits, bias, tok.hidden_states, tok.hidden_states_scale, W.gemm1_weights, W.gemm1_weights_scale,
+                     W.gemm2_weights, W.gemm2_weights_scale, 0, RSF)
+    assert pkg.op.kernel_status() == 0
+    assert_output_close(out, ref.output, ref.output_f32)
+    assert float(out[sum(counts):].float().abs().max()) == 0.0
 
 
 @pytest.mark.parametrize("T,seed,skew,offset", [(4096, 0, False, 0), (1100, 3, True, 0), (6000, 5, False, 96)])
