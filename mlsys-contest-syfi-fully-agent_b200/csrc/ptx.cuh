@@ -65,37 +65,37 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
                : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+// One poll by all 32 lanes of a converged warp: true in every lane if the phase is complete for all of them.
+__device__ __forceinline__ bool mbar_try_wait_all(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
+      "vote.sync.all.pred q, p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(done)
       : "r"(bar), "r"(parity)
       : "memory");
   return done != 0;
 }
 
-// Bounded wait.  `abort_flag` lives in shared memory and is shared by every role
-// of the CTA: the first role that times out sets it, the others see it on their
-// next poll and leave too.
+// Bounded wait of a whole converged warp.  Every lane gets the same answer: what follows a wait in the kernels (elect.sync,
+// ballots, shuffles, tcgen05.ld) needs all 32 lanes, and lanes that left on a timeout while others saw the phase
+// complete would be waited for without a limit.  `abort_flag` lives in shared memory and is shared by every role of the
+// CTA: the first warp that times out sets it, the others see it on a later poll and leave too.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
   uint64_t t0 = 0;
   uint32_t spins = 0;
-  while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
+  while (!mbar_try_wait_all(bar, parity)) {
     if ((++spins & 0x3Fu) == 0) {
       const uint64_t t = globaltimer_ns();
       if (t0 == 0) t0 = t;
-      else if (t - t0 > MOE_WAIT_LIMIT_NS) {
-        *abort_flag = 1;
-        return false;
-      }
+      const bool late = t - t0 > MOE_WAIT_LIMIT_NS;
+      if (late) *abort_flag = 1;
+      if (__any_sync(0xFFFFFFFFu, late || *abort_flag != 0)) return false;
     }
   }
+  return true;
 }
 
 // ----------------------------------------------------------------------------- cp.async (4 bytes per thread)

@@ -18,15 +18,32 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 
 
-def test_bounded_waits_run_out_and_the_context_stays_usable(pkg, tmp_path):
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc is not available to build the probe")
-    lib_path = str(tmp_path / "libwait_probe.so")
+    lib_path = str(tmp_path_factory.mktemp("probe") / "libwait_probe.so")
     subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17", "-shared", "-Xcompiler",
                     "-fPIC", "-I", os.path.join(ROOT, "mlsys-contest-syfi-fully-agent_b200", "csrc"), "-o", lib_path,
                     os.path.join(HERE, "wait_probe.cu")], check=True)
-    lib = ctypes.CDLL(lib_path)
+    return ctypes.CDLL(lib_path)
+
+
+@pytest.mark.parametrize("split", [0, 1, 16, 31, 32])
+def test_all_lanes_of_a_waiting_warp_get_the_same_answer(lib, split):
+    """`split` lanes wait on a phase that is complete, the rest on one that never completes: the wait has succeeded only
+    if it has for all 32.  (The kernels run elect.sync, ballots and tcgen05.ld behind a wait: a lane that was told
+    something else than its neighbours would be waited for without a limit.)"""
+    res = torch.full((32,), -1, dtype=torch.int32, device="cuda")
+    fn = lib.moe_test_mbarrier_lanes
+    fn.restype, fn.argtypes = ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    assert fn(res.data_ptr(), split, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert res.tolist() == [1 if split == 32 else 0] * 32
+
+
+def test_bounded_waits_run_out_and_the_context_stays_usable(pkg, lib):
     lib.moe_test_wait_timeouts.restype = ctypes.c_int
     lib.moe_test_wait_timeouts.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
     dev = torch.device("cuda", 0)

@@ -19,8 +19,9 @@ __global__ void grid_barrier_probe(unsigned int* word2, int* status, unsigned in
   if (!moe::grid_barrier_wait(word2, tag, gridDim.x + 1)) atomicOr(status, moe::kErrGemm1Timeout);
 }
 
-// The pipeline's mbarrier wait on a phase that no arrival or TMA transaction ever completes; a second
-// warp sees the CTA-wide abort flag and leaves as well.
+// The pipeline's mbarrier wait (a whole warp waits) on a phase that no arrival or TMA transaction ever completes; a
+// second warp sees the CTA-wide abort flag and leaves as well.  Both warps then elect a lane, as the kernels do behind
+// a wait.
 __global__ void mbarrier_probe(int* status) {
   __shared__ uint64_t bar;
   __shared__ int abort_flag;
@@ -30,11 +31,26 @@ __global__ void mbarrier_probe(int* status) {
     moe::fence_mbar_init();
   }
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) {
-    if (!moe::mbar_wait(moe::smem_u32(&bar), 0, &abort_flag)) atomicOr(status, moe::kErrGemm2Timeout);
-  }
+  if (!moe::mbar_wait(moe::smem_u32(&bar), 0, &abort_flag) && moe::elect_one()) atomicOr(status, moe::kErrGemm2Timeout);
   __syncthreads();
   if (threadIdx.x == 0 && abort_flag) atomicOr(status, 0x200);
+}
+
+// The answer of a warp whose lanes see different phases: lanes below `split` wait on a barrier that is complete, the
+// others on one that never is.  results[lane] = what the lane was told (0 / 1).  No collective follows, so lanes that
+// were told different things would still all leave.
+__global__ void mbarrier_lanes_probe(int* results, int split) {
+  __shared__ uint64_t bar[2];
+  __shared__ int abort_flag;
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int i = 0; i < 2; ++i) moe::mbar_init(moe::smem_u32(&bar[i]), 1);
+    moe::fence_mbar_init();
+    moe::mbar_arrive(moe::smem_u32(&bar[0]));
+  }
+  __syncthreads();
+  const int lane = static_cast<int>(threadIdx.x);
+  results[lane] = moe::mbar_wait(moe::smem_u32(&bar[lane < split ? 0 : 1]), 0, &abort_flag) ? 1 : 0;
 }
 
 }  // namespace
@@ -44,5 +60,11 @@ extern "C" int moe_test_wait_timeouts(int* status_dev, unsigned int* word_dev, v
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   grid_barrier_probe<<<4, 32, 0, stream>>>(word_dev, status_dev, 0x5EEDu);
   mbarrier_probe<<<1, 64, 0, stream>>>(status_dev);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// results_dev: 32 ints.  Lanes below `split` wait for something that has happened, the others for something that never does.
+extern "C" int moe_test_mbarrier_lanes(int* results_dev, int split, void* stream_v) {
+  mbarrier_lanes_probe<<<1, 32, 0, static_cast<cudaStream_t>(stream_v)>>>(results_dev, split);
   return static_cast<int>(cudaGetLastError());
 }
