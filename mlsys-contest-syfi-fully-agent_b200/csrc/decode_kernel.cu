@@ -425,7 +425,7 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
                   }
                 }
               }
-              if (!grid_barrier_wait(bar, call_tag, 2 * n_ctas)) { *abort_flag = 1; ok = false; break; }
+              if (!grid_barrier_wait_warp(bar, call_tag, 2 * n_ctas)) { *abort_flag = 1; ok = false; break; }
               fence_proxy_async_global();   // the planes were written with ordinary stores by other SMs
               ready = true;
             }

@@ -43,6 +43,18 @@ def test_all_lanes_of_a_waiting_warp_get_the_same_answer(lib, split):
     assert res.tolist() == [1 if split == 32 else 0] * 32
 
 
+@pytest.mark.parametrize("split", [0, 1, 31, 32])
+def test_all_lanes_at_the_grid_barrier_get_the_same_answer(lib, split):
+    """The decode kernel's TMA producer waits at the grid barrier with its whole warp: the same of that wait."""
+    res = torch.full((32,), -1, dtype=torch.int32, device="cuda")
+    word = torch.zeros(2, dtype=torch.int32, device="cuda")
+    fn = lib.moe_test_grid_barrier_lanes
+    fn.restype, fn.argtypes = ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    assert fn(res.data_ptr(), word.data_ptr(), split, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert res.tolist() == [1 if split == 32 else 0] * 32
+
+
 def test_bounded_waits_run_out_and_the_context_stays_usable(pkg, lib):
     lib.moe_test_wait_timeouts.restype = ctypes.c_int
     lib.moe_test_wait_timeouts.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]

@@ -19,6 +19,18 @@ __global__ void grid_barrier_probe(unsigned int* word2, int* status, unsigned in
   if (!moe::grid_barrier_wait(word2, tag, gridDim.x + 1)) atomicOr(status, moe::kErrGemm1Timeout);
 }
 
+// The producer's form of that wait, by a warp whose lanes ask for different targets: lanes below `split` for the one
+// arrival there is, the others for one more.  results[lane] = what the lane was told; no collective follows.
+__global__ void grid_barrier_lanes_probe(unsigned int* word2, int* results, int split, unsigned int tag) {
+  const int lane = static_cast<int>(threadIdx.x);
+  if (lane == 0) {
+    moe::grid_barrier_init(word2, tag);
+    moe::grid_barrier_arrive(word2);
+  }
+  __syncwarp();
+  results[lane] = moe::grid_barrier_wait_warp(word2, tag, lane < split ? 1u : 2u) ? 1 : 0;
+}
+
 // The pipeline's mbarrier wait (a whole warp waits) on a phase that no arrival or TMA transaction ever completes; a
 // second warp sees the CTA-wide abort flag and leaves as well.  Both warps then elect a lane, as the kernels do behind
 // a wait.
@@ -66,5 +78,11 @@ extern "C" int moe_test_wait_timeouts(int* status_dev, unsigned int* word_dev, v
 // results_dev: 32 ints.  Lanes below `split` wait for something that has happened, the others for something that never does.
 extern "C" int moe_test_mbarrier_lanes(int* results_dev, int split, void* stream_v) {
   mbarrier_lanes_probe<<<1, 32, 0, static_cast<cudaStream_t>(stream_v)>>>(results_dev, split);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// The same of the decode kernel's grid barrier; word_dev: two uints (any contents).
+extern "C" int moe_test_grid_barrier_lanes(int* results_dev, unsigned int* word_dev, int split, void* stream_v) {
+  grid_barrier_lanes_probe<<<1, 32, 0, static_cast<cudaStream_t>(stream_v)>>>(word_dev, results_dev, split, 0x5EEDu);
   return static_cast<int>(cudaGetLastError());
 }
