@@ -15,6 +15,7 @@
 
 #include "../../include/moe_b200.h"
 #include "kernels.h"
+#include "map_cache.h"
 
 namespace moe {
 namespace {
@@ -86,29 +87,7 @@ struct DeviceState {
 std::mutex g_mu;
 DeviceState g_dev[16];
 
-struct MapKey {
-  const void* ptr;
-  uint32_t rank;
-  uint64_t dims[4];
-  uint64_t strides[3];
-  uint32_t box[4];
-  bool operator==(const MapKey& o) const {
-    if (ptr != o.ptr || rank != o.rank) return false;
-    for (uint32_t i = 0; i < rank; ++i)
-      if (dims[i] != o.dims[i] || box[i] != o.box[i]) return false;
-    for (uint32_t i = 0; i + 1 < rank; ++i)
-      if (strides[i] != o.strides[i]) return false;
-    return true;
-  }
-};
-constexpr int kMapCache = 64;   // a call uses up to 12 maps; several batch-size classes stay cached side by side
-struct MapEntry {
-  MapKey key;
-  CUtensorMap map;
-  bool used;
-};
-MapEntry g_maps[kMapCache];
-int g_map_next = 0;
+MapCache<CUtensorMap> g_maps;   // under g_mu
 
 int ensure_device(DeviceState** out) {
   int dev = 0;
@@ -141,11 +120,7 @@ int ensure_device(DeviceState** out) {
 // u8 tensor map with the 128-byte swizzle; dims / box innermost first, strides in bytes for dims 1..rank-1.
 int get_map(DeviceState* d, const MapKey& key, CUtensorMap* out) {
   std::lock_guard<std::mutex> lk(g_mu);
-  for (auto& e : g_maps)
-    if (e.used && e.key == key) {
-      *out = e.map;
-      return MOE_B200_OK;
-    }
+  if (g_maps.find(key, out)) return MOE_B200_OK;
   cuuint64_t dims[4], strides[3];
   cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
   for (uint32_t i = 0; i < key.rank; ++i) { dims[i] = key.dims[i]; box[i] = key.box[i]; }
@@ -158,11 +133,7 @@ int get_map(DeviceState* d, const MapKey& key, CUtensorMap* out) {
     g_last_cuda_error = 100000 + static_cast<int>(r);
     return MOE_B200_ECUDA;
   }
-  MapEntry& e = g_maps[g_map_next];
-  g_map_next = (g_map_next + 1) % kMapCache;
-  e.key = key;
-  e.map = m;
-  e.used = true;
+  g_maps.insert(key, m);
   *out = m;
   return MOE_B200_OK;
 }
