@@ -12,6 +12,8 @@ from __future__ import annotations
 import json
 import os
 
+from . import build
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
@@ -21,9 +23,8 @@ DEFINITION = "moe_fp8_block_scale_ds_routing_topk8_ng8_kg4_e32_h7168_i2048"
 AUTHOR = "b200-native"
 ENTRY_POINT = "tvm_ffi_shim.cu::run"
 
-SOURCE_FILES = ["tvm_ffi_shim.cu", "launcher.cu", "route_permute.cu", "grouped_gemm.cu", "decode_kernel.cu", "swiglu_combine.cu",
-                "static_entry.cu", "quantize.cu", "ep_push.cu", "kernels.h", "moe_layout.h", "map_cache.h", "ptx.cuh", "route_device.cuh",
-                "epilogue_device.cuh", "gemm_common.cuh"]
+# everything the library is built from, the tvm-ffi shim first
+SOURCE_FILES = ["tvm_ffi_shim.cu"] + build.SOURCES + [h for h in build.HEADERS if not h.startswith("..")]
 
 
 def flattened_sources():

@@ -42,3 +42,10 @@ def test_flattened_directory_compiles(pkg, tmp_path):
     subprocess.run(cmd, check=True, cwd=str(src))
     syms = subprocess.run(["nm", "-D", str(out)], check=True, capture_output=True, text=True).stdout
     assert "__tvm_ffi_run" in syms
+    assert not [s for s in syms.splitlines() if " U _ZN3moe" in s]      # and it can be loaded
+
+
+def test_every_source_of_the_library_is_packed(pkg):
+    """A missing source still links as a shared library and fails only when the harness loads it."""
+    assert set(pkg.build.SOURCES) <= set(pkg.packaging.SOURCE_FILES)
+    assert {h for h in pkg.build.HEADERS if not h.startswith("..")} <= set(pkg.packaging.SOURCE_FILES)
