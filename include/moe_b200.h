@@ -171,7 +171,9 @@ int moe_fp8_block_scale_last_cuda_error(void);
 /* Where the intermediate arrays of the last call live inside the workspace
  * (byte offsets), for parity tests that compare selection, permutation and
  * per-stage results with the definition.  Mirrors the reference's process-global
- * Workspace (moe.cu:2511-2589), owned by the caller instead. */
+ * Workspace (moe.cu:2511-2589), owned by the caller instead.  For T > 16 the two scale tables
+ * are K-block-major.  They used to be [rows_cap, 56] and [rows_cap, 16] for every T, under the
+ * names a_scale_rows and c_scale: a reader of those has to swap its indices, hence the new names. */
 typedef struct moe_b200_layout {
   int32_t T, rows_cap, slab_rows, n_terms;
   uint64_t sched;        /* moe_b200_sched                                   */
@@ -182,10 +184,10 @@ typedef struct moe_b200_layout {
   uint64_t perm_weight;  /* f32 [n_sel]                                      */
   uint64_t tok_rows;     /* i32 [T, 8] rows of each token, ascending expert  */
   uint64_t a_packed;     /* e4m3 [rows_cap, 7168] permuted activations       */
-  uint64_t a_scale_rows; /* f32 [56, rows_cap] block scales of the permuted rows */
+  uint64_t a_scale_kb;   /* f32 [56, rows_cap] block scales of the permuted rows (T > 16) */
   uint64_t g1;           /* f32 [split1][n_sel_pad, 4096] GEMM1 slabs        */
   uint64_t cq;           /* e4m3 [n_terms][rows_cap, 2048] SwiGLU planes     */
-  uint64_t c_scale;      /* f32 [rows_cap, 16]                               */
+  uint64_t plane_scale;  /* f32 [16, rows_cap] (T <= 16: [rows_cap, 16]) scales of the SwiGLU planes */
   uint64_t o;            /* f32 [split2][n_sel_pad, 7168] GEMM2 slabs        */
   uint64_t acc32;        /* f32 [T, 7168] output accumulator (fast combine)  */
   uint64_t tile_cnt;     /* i32 [T, 56] arrivals per (token, column tile)    */

@@ -44,9 +44,9 @@ __device__ __forceinline__ void split_e4m3_terms(float r, uint8_t* t) {
 }
 
 // SwiGLU of 4 columns per lane of one (row, 128-column block), split of the result into kNTerms e4m3
-// planes with one power-of-two scale for the block.
+// planes with one power-of-two scale for the block, stored to *scale_out.
 __device__ __forceinline__ void swiglu_finish_block(const float4 x1, const float4 x2, int row, int kb, int lane, uint8_t* cq,
-                                                    float* c_scale, float* c_scale_kb, int rows_cap) {
+                                                    float* scale_out, int rows_cap) {
   float c[4];
   c[0] = swiglu_value(x1.x, x2.x);
   c[1] = swiglu_value(x1.y, x2.y);
@@ -72,19 +72,16 @@ __device__ __forceinline__ void swiglu_finish_block(const float4 x1, const float
   for (int t = 0; t < kNTerms; ++t)
     *reinterpret_cast<uint32_t*>(cq + (static_cast<size_t>(t) * rows_cap + row) * kI + kb * kBlock + lane * 4) =
         packed[t];
-  if (lane == 0) {
-    c_scale[static_cast<size_t>(row) * kKB2 + kb] = scale;
-    if (c_scale_kb) c_scale_kb[static_cast<size_t>(kb) * rows_cap + row] = scale;
-  }
+  if (lane == 0) *scale_out = scale;
 }
 
 // SwiGLU + e4m3 split of NB consecutive 128-column blocks of one row by one warp; lane owns 4
 // columns of each block.  `g1` points at the first split-K slab; slabs are `slab` floats apart.
 // All loads of the NB blocks are issued before any arithmetic (memory-level parallelism), and they
-// bypass L1 (the slabs may have been written by other SMs in the same kernel).
+// bypass L1 (the slabs may have been written by other SMs in the same kernel).  The scales go out K-block-major.
 template <int NB>
 __device__ __forceinline__ void swiglu_split_blocks(const float* g1, size_t slab, int split, int row, int kb0, int lane,
-                                                    uint8_t* cq, float* c_scale, float* c_scale_kb, int rows_cap) {
+                                                    uint8_t* cq, float* c_scale, int rows_cap) {
   float4 x1[NB], x2[NB];
 #pragma unroll
   for (int b = 0; b < NB; ++b) x1[b] = x2[b] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -117,11 +114,13 @@ __device__ __forceinline__ void swiglu_split_blocks(const float* g1, size_t slab
     }
   }
 #pragma unroll
-  for (int b = 0; b < NB; ++b) swiglu_finish_block(x1[b], x2[b], row, kb0 + b, lane, cq, c_scale, c_scale_kb, rows_cap);
+  for (int b = 0; b < NB; ++b)
+    swiglu_finish_block(x1[b], x2[b], row, kb0 + b, lane, cq, c_scale + static_cast<size_t>(kb0 + b) * rows_cap + row, rows_cap);
 }
 
 // The same for one block whose two halves have their own numbers of slabs (balanced partition of the
-// decode kernel): x1 = sum of n1 slabs, x2 = sum of n2 slabs, each in slab order.
+// decode kernel): x1 = sum of n1 slabs, x2 = sum of n2 slabs, each in slab order.  The scales are row-major here: a few
+// rows' sixteen scales are a line or two (K-block-major, a call at T = 1 takes 0.25 us more).
 __device__ __forceinline__ void swiglu_split_unit2(const float* g1, size_t slab, int n1, int n2, int row, int kb, int lane,
                                                    uint8_t* cq, float* c_scale, int rows_cap) {
   constexpr int kMax = 8;
@@ -138,7 +137,7 @@ __device__ __forceinline__ void swiglu_split_unit2(const float* g1, size_t slab,
     if (s < n1) { x1.x += u[s].x; x1.y += u[s].y; x1.z += u[s].z; x1.w += u[s].w; }
     if (s < n2) { x2.x += v[s].x; x2.y += v[s].y; x2.z += v[s].z; x2.w += v[s].w; }
   }
-  swiglu_finish_block(x1, x2, row, kb, lane, cq, c_scale, nullptr, rows_cap);
+  swiglu_finish_block(x1, x2, row, kb, lane, cq, c_scale + static_cast<size_t>(row) * kKB2 + kb, rows_cap);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

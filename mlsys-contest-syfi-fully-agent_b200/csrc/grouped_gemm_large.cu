@@ -396,11 +396,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
             dst[0] = make_uint4(pk[t][0], pk[t][1], pk[t][2], pk[t][3]);
             dst[1] = make_uint4(pk[t][4], pk[t][5], pk[t][6], pk[t][7]);
           }
-          if (cg == 0) {
-            const float scale = __uint_as_float(static_cast<uint32_t>(ex + 127) << 23);
-            a.c_scale[static_cast<size_t>(row) * kKB2 + w.j] = scale;
-            a.c_scale_kb[static_cast<size_t>(w.j) * a.rows_cap + row] = scale;
-          }
+          if (cg == 0) a.c_scale[static_cast<size_t>(w.j) * a.rows_cap + row] = __uint_as_float(static_cast<uint32_t>(ex + 127) << 23);
         }
       } else {
         const int tile = 2 * w.j + (cg >> 1);     // the 128-row weight block of this thread's columns

@@ -94,8 +94,7 @@ struct GemmArgs {
   int ctas, rows_cap, slab_rows;
   int* topk_idx; float* topk_w; uint32_t* local_mask;
   int* perm_token; float* perm_weight; int* tok_rows;
-  uint8_t* cq; float* c_scale;  // SwiGLU planes and their scales [rows_cap, 16]
-  float* c_scale_kb;            // the scales again as [16, rows_cap] (GEMM2's b_scale); null in the decode kernel
+  uint8_t* cq; float* c_scale;  // SwiGLU planes and their scales, [16, rows_cap] (decode kernel: [rows_cap, 16])
   uint16_t* out_bf16;           // final output
   uint16_t* const* out_rows;    // optional per-token destinations instead of out_bf16 (may be peer memory)
   // ---- only read by the large-batch GEMM2 with the fused combine (grouped_gemm_large.cu)
@@ -107,8 +106,7 @@ struct SwigluArgs {
   const MoeSched* sched;
   const float* g1;              // slabs [split1][n_sel_pad, 4096]
   uint8_t* cq;                  // [kNTerms][rows_cap, 2048] e4m3 planes
-  float* c_scale;               // [rows_cap, 16] power-of-two plane scale per 128 block
-  float* c_scale_kb;            // the same, [16, rows_cap]
+  float* c_scale;               // [16, rows_cap] power-of-two plane scale per 128 block, K-block-major like a_scale
   int rows_cap;
 };
 

@@ -209,10 +209,10 @@ extern "C" int moe_fp8_block_scale_layout(int T, moe_b200_layout* out) {
   out->perm_weight = L.perm_weight;
   out->tok_rows = L.tok_rows;
   out->a_packed = L.a_packed;
-  out->a_scale_rows = L.a_scale_rows;
+  out->a_scale_kb = L.a_scale_kb;
   out->g1 = L.g1;
   out->cq = L.cq;
-  out->c_scale = L.c_scale;
+  out->plane_scale = L.plane_scale;
   out->o = L.o;
   out->acc32 = L.acc32;
   out->tile_cnt = L.tile_cnt;
@@ -253,11 +253,10 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
   int* tok_rows = reinterpret_cast<int*>(ws + L.tok_rows);
   int* chunk_base = reinterpret_cast<int*>(ws + L.chunk_base);
   uint8_t* a_packed = ws + L.a_packed;
-  float* a_scale = reinterpret_cast<float*>(ws + L.a_scale_rows);
+  float* a_scale = reinterpret_cast<float*>(ws + L.a_scale_kb);
   float* g1 = reinterpret_cast<float*>(ws + L.g1);
   uint8_t* cq = ws + L.cq;
-  float* c_scale = reinterpret_cast<float*>(ws + L.c_scale);
-  float* c_scale_kb = reinterpret_cast<float*>(ws + L.c_scale_kb);
+  float* c_scale = reinterpret_cast<float*>(ws + L.plane_scale);
   float* o = reinterpret_cast<float*>(ws + L.o);
   float* acc32 = reinterpret_cast<float*>(ws + L.acc32);
   int* tile_cnt = reinterpret_cast<int*>(ws + L.tile_cnt);
@@ -326,9 +325,9 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
 
   GemmArgs g1a{};
   g1a.sched = sched; g1a.w_scale = gemm1_weights_scale; g1a.b_scale = a_scale; g1a.out = g1;
-  g1a.rows_cap = L.rows_cap; g1a.cq = cq; g1a.c_scale = c_scale; g1a.c_scale_kb = c_scale_kb;
+  g1a.rows_cap = L.rows_cap; g1a.cq = cq; g1a.c_scale = c_scale;
   GemmArgs g2a{};
-  g2a.sched = sched; g2a.w_scale = gemm2_weights_scale; g2a.b_scale = c_scale_kb; g2a.out = o;
+  g2a.sched = sched; g2a.w_scale = gemm2_weights_scale; g2a.b_scale = c_scale; g2a.out = o;
   g2a.rows_cap = L.rows_cap; g2a.perm_token = perm_token; g2a.perm_weight = perm_weight; g2a.local_mask = local_mask;
   g2a.acc32 = acc32; g2a.tile_cnt = tile_cnt; g2a.out_bf16 = output; g2a.out_rows = output_rows;
 
@@ -374,7 +373,7 @@ static int run_impl(const float* routing_logits, const uint16_t* routing_bias, c
     g_launches += 1;
     stage_mark(3, stream);
 
-    SwigluArgs sa{sched, g1, cq, c_scale, c_scale_kb, L.rows_cap};
+    SwigluArgs sa{sched, g1, cq, c_scale, L.rows_cap};
     launch_swiglu_split(sa, T, stream);
     MOE_CUDA(cudaGetLastError());
     g_launches += 1;

@@ -63,7 +63,7 @@ struct WorkspaceLayout {
   int rows_cap;        // capacity in rows: 8*T rounded up to 128
   int slab_rows;       // rows of the fp32 slab areas: max(rows_cap, kMinSlabRows)
   size_t sched, topk_idx, topk_w, local_mask, perm_token, perm_weight, tok_rows, chunk_base;
-  size_t a_packed, a_scale_rows, g1, cq, c_scale, c_scale_kb, o;
+  size_t a_packed, a_scale_kb, g1, cq, plane_scale, o;
   size_t acc32, tile_cnt;   // fused combine of the large-batch GEMM2: fp32 output accumulator and arrival counters
   size_t total;
 };
@@ -92,11 +92,10 @@ inline WorkspaceLayout make_layout(int T) {
   L.tok_rows = take(Tz * kTopK * 4);
   L.chunk_base = take((Tz + 31) / 32 * kELocal * 4);   // first row of every (32-token chunk, expert)
   L.a_packed = take(static_cast<size_t>(L.rows_cap) * kH);
-  L.a_scale_rows = take(static_cast<size_t>(L.rows_cap) * kKB1 * 4);
+  L.a_scale_kb = take(static_cast<size_t>(L.rows_cap) * kKB1 * 4);
   L.g1 = take(static_cast<size_t>(L.slab_rows) * k2I * 4);
   L.cq = take(static_cast<size_t>(kNTerms) * L.rows_cap * kI);
-  L.c_scale = take(static_cast<size_t>(L.rows_cap) * kKB2 * 4);
-  L.c_scale_kb = take(static_cast<size_t>(L.rows_cap) * kKB2 * 4);   // the same scales, K-block-major
+  L.plane_scale = take(static_cast<size_t>(L.rows_cap) * kKB2 * 4);
   L.o = take(static_cast<size_t>(L.slab_rows) * kH * 4);
   L.acc32 = take(Tz * kH * 4);
   L.tile_cnt = take(Tz * kMT2 * 4);

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) swiglu_split_kernel(SwigluArgs a) {
   const long long wstride = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   for (long long b = blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5); b < nunit; b += wstride)
     swiglu_split_blocks<kNB>(a.g1, slab, split, static_cast<int>(b / (kKB2 / kNB)),
-                             static_cast<int>(b % (kKB2 / kNB)) * kNB, lane, a.cq, a.c_scale, a.c_scale_kb, a.rows_cap);
+                             static_cast<int>(b % (kKB2 / kNB)) * kNB, lane, a.cq, a.c_scale, a.rows_cap);
 }
 
 // One 256-thread block per token (grid-stride over tokens).

@@ -46,7 +46,7 @@ class Layout(ctypes.Structure):
     _fields_ = [("T", ctypes.c_int32), ("rows_cap", ctypes.c_int32), ("slab_rows", ctypes.c_int32),
                 ("n_terms", ctypes.c_int32)] + \
                [(n, ctypes.c_uint64) for n in ("sched", "topk_idx", "topk_w", "local_mask", "perm_token",
-                                               "perm_weight", "tok_rows", "a_packed", "a_scale_rows", "g1", "cq", "c_scale", "o",
+                                               "perm_weight", "tok_rows", "a_packed", "a_scale_kb", "g1", "cq", "plane_scale", "o",
                                                "acc32", "tile_cnt", "total")]
 
 

@@ -40,10 +40,18 @@ def test_workspace_size_and_layout(loader):
         L = loader.layout(T)
         assert L.total == n and L.rows_cap >= 8 * T and L.rows_cap % 128 == 0
         offs = [L.sched, L.topk_idx, L.topk_w, L.local_mask, L.perm_token, L.perm_weight, L.tok_rows,
-                L.a_packed, L.a_scale_rows, L.g1, L.cq, L.c_scale, L.o]
+                L.a_packed, L.a_scale_kb, L.g1, L.cq, L.plane_scale, L.o]
         assert offs == sorted(offs) and all(o % 1024 == 0 for o in offs) and offs[-1] < n
     assert loader.workspace_bytes(-1) == 0
     assert ctypes.sizeof(loader.Sched) == (16 + 32 + 33 + 33 + 33) * 4
+
+
+@pytest.mark.parametrize("T,size", [(1, 94076672), (16, 94851072), (17, 96643328), (512, 266786304), (1024, 533571072),
+                                    (1025, 541138688), (4096, 2134279680), (14107, 7353000448), (16384, 8537114112)])
+def test_a_workspace_sized_by_an_earlier_release_is_large_enough(loader, T, size):
+    """`size` is what ..._workspace_bytes(T) returned when the scale tables were row-major: a caller that stored it is
+    not refused."""
+    assert loader.workspace_bytes(T) <= size
 
 
 def test_bad_arguments_are_rejected_without_a_device(loader):

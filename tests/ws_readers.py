@@ -34,6 +34,12 @@ def _sum_slabs(arr, offset, sched, gemm, pad, width):
     return res
 
 
+def _plane_scales(ws, L, n_sel):
+    """f32 [n_sel, 16]: the scales of the SwiGLU planes that GEMM2 multiplied by (K-block-major above 16 tokens)."""
+    s = ws.view(L.plane_scale, L.rows_cap * 16 * 4).view(torch.float32)
+    return s.view(L.rows_cap, 16)[:n_sel].clone() if L.T <= 16 else s.view(16, L.rows_cap)[:, :n_sel].t().contiguous()
+
+
 def intermediates(pkg, T: int, workspace=None, device=None, stages: bool = True) -> dict:
     """Host copies of the selection / permutation / per-stage arrays the last
     call with ``T`` tokens left in the workspace.  ``stages=False`` skips the fp32 / fp8 per-stage
@@ -64,7 +70,7 @@ def intermediates(pkg, T: int, workspace=None, device=None, stages: bool = True)
         out["g1"] = _sum_slabs(arr, L.g1, sched, 1, pad, 4096)[:n_sel].cpu()
         out["o"] = _sum_slabs(arr, L.o, sched, 2, pad, H)[:n_sel].cpu()
         cq = arr(L.cq, L.n_terms * L.rows_cap * I, torch.float8_e4m3fn, (L.n_terms, L.rows_cap, I))[:, :n_sel]
-        cs = arr(L.c_scale, L.rows_cap * 16 * 4, torch.float32, (L.rows_cap, 16))[:n_sel]
+        cs = _plane_scales(ws, L, n_sel)
         c = cq.to(torch.float32).sum(dim=0).view(n_sel, 16, 128) * cs.unsqueeze(2)
         out["c"] = c.view(n_sel, I).cpu()
         out["a_packed"] = arr(L.a_packed, n_sel * H, torch.uint8, (n_sel, H)).cpu()
@@ -81,5 +87,5 @@ def swiglu_planes(pkg, T: int, workspace=None, device=None):
     L = loader.layout(T)
     n_sel = op.read_schedule(T, workspace, device).n_sel
     cq = ws.view(L.cq, L.n_terms * L.rows_cap * I).view(L.n_terms, L.rows_cap, I)[:, :n_sel].clone()
-    cs = ws.view(L.c_scale, L.rows_cap * 16 * 4).view(torch.float32).view(L.rows_cap, 16)[:n_sel].clone()
+    cs = _plane_scales(ws, L, n_sel)
     return cq, cs
