@@ -174,7 +174,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
     aux->abort = 0;
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(smem_u32(&aux->full[s]), 1 + 32);     // the TMA producer and the 32 lanes of the scale warp
-      mbar_init(smem_u32(&aux->done[s]), 1);
+      mbar_init(smem_u32(&aux->done[s]), 2);          // the commit and the issuer's own arrival
     }
     for (int b = 0; b < C::NBUF; ++b) mbar_init(smem_u32(&aux->tempty[b]), kEpiWarps);
     fence_mbar_init();
@@ -284,6 +284,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
               }
             }
             umma_commit(done_base + stage * 8);
+            // The promotion warps read the stage's scales behind `done` and never wait on `full`.  The commit orders the
+            // UMMAs; this arrival releases what the issuer acquired with `full`, the copied scales among it.
+            mbar_arrive(done_base + stage * 8);
           }
         }
       }

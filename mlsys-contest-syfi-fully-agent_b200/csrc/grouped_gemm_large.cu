@@ -171,7 +171,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     for (int s = 0; s < C::WS; ++s) mbar_init(smem_u32(&aux->wfull[s]), 1 + 32);   // the producer and the scale warp's lanes
     for (int s = 0; s < C::PS; ++s) {
       mbar_init(smem_u32(&aux->pfull[s]), 1);
-      mbar_init(smem_u32(&aux->pdone[s]), 1);
+      mbar_init(smem_u32(&aux->pdone[s]), 2);      // the commit and the issuer's own arrival
     }
     for (int b = 0; b < C::NBUF; ++b) mbar_init(smem_u32(&aux->tempty[b]), kLEpiWarps);
     mbar_init(smem_u32(&aux->esync), kLEpiThreads);
@@ -301,6 +301,9 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
                 for (int k4 = 0; k4 < 4; ++k4)   // +32 bytes of K inside the 128-byte swizzle atom = +2 encoded units
                   umma_f8(d, tdesc + 2 * k4, wdesc + 2 * k4, idesc, (t | k4) != 0 ? 1u : 0u);
                 umma_commit(pdone_base + pp.i * 8);
+                // the promotion warps read the K-block's scales behind `pdone` alone: this arrival releases to them what
+                // the issuer acquired with `wfull` (see grouped_gemm.cu)
+                mbar_arrive(pdone_base + pp.i * 8);
               }
             }
             if (!ok) break;
