@@ -83,8 +83,8 @@ __device__ __forceinline__ bool mbar_try_wait_all(uint32_t bar, uint32_t parity)
 // ballots, shuffles, tcgen05.ld) needs all 32 lanes, and lanes that left on a timeout while others saw the phase
 // complete would be waited for without a limit.  `abort_flag` lives in shared memory and is shared by every role of the
 // CTA: the first warp that times out sets it, the others see it on a later poll and leave too.
-// The first poll stands in front of the loop: with it inside, the large-batch kernels take 1.5 % longer (T = 14107: 1202
-// against 1194 us; 1201 with a wait that does not vote).
+// The first poll stands in front of the loop: a call at T = 14107 takes 0.6 % less than with a wait that does not vote,
+// and 1.5 % more if the first poll is the loop's.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait_all(bar, parity)) return true;
   uint64_t t0 = 0;
@@ -109,6 +109,19 @@ __device__ __forceinline__ void cp_async4(uint32_t dst_smem, const void* src) {
 }
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// Teardown of a CTA that has given up a wait, before it frees its TMEM and returns: its own copies and UMMAs may still be
+// in flight, and they write shared memory and TMEM that belong to somebody else once it has left.  The barriers they
+// report to can be half armed (a role that left early has not arrived), so this waits for time and not for them:
+// MOE_ABORT_SETTLE_NS, hundreds of times what a load or a stage of UMMAs takes.
+#ifndef MOE_ABORT_SETTLE_NS
+#define MOE_ABORT_SETTLE_NS 1000000ull
+#endif
+__device__ __forceinline__ void settle_after_abort() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  const uint64_t t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < MOE_ABORT_SETTLE_NS) __nanosleep(1000);
 }
 
 // ----------------------------------------------------------------------------- TMA (tiled, no multicast)

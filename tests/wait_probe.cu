@@ -45,6 +45,7 @@ __global__ void mbarrier_probe(int* status) {
   __syncthreads();
   if (!moe::mbar_wait(moe::smem_u32(&bar), 0, &abort_flag) && moe::elect_one()) atomicOr(status, moe::kErrGemm2Timeout);
   __syncthreads();
+  if (abort_flag) moe::settle_after_abort();
   if (threadIdx.x == 0 && abort_flag) atomicOr(status, 0x200);
 }
 
