@@ -91,25 +91,8 @@ __device__ __forceinline__ void grid_barrier_init(unsigned int* word2, unsigned 
   atomicExch(reinterpret_cast<unsigned long long*>(word2), static_cast<unsigned long long>(tag) << 32);
 }
 
-__device__ __forceinline__ bool grid_barrier(unsigned int* word2, unsigned int tag, unsigned int n) {
-  unsigned long long* word = reinterpret_cast<unsigned long long*>(word2);
-  __threadfence();
-  const uint64_t t0 = globaltimer_ns();
-  unsigned int spins = 0;
-  while (static_cast<unsigned int>(*reinterpret_cast<volatile unsigned long long*>(word) >> 32) != tag)
-    if ((++spins & 0xFFu) == 0 && globaltimer_ns() - t0 > MOE_WAIT_LIMIT_NS) return false;
-  atomicAdd(word, 1ull);
-  while (true) {
-    const unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(word);
-    if (static_cast<unsigned int>(v) >= n) break;
-    if ((++spins & 0xFFu) == 0 && globaltimer_ns() - t0 > MOE_WAIT_LIMIT_NS) return false;
-  }
-  __threadfence();
-  return true;
-}
-
-// The same barrier in separate steps, for a word that serves several successive barriers of one launch
-// (the k-th is complete at k * gridDim.x arrivals) and for waiters that do not arrive (a TMA producer).
+// In separate steps, for a word that serves several successive barriers of one launch (the k-th is complete at
+// k * gridDim.x arrivals) and for waiters that do not arrive (a TMA producer).
 // One thread per CTA arrives, after a CTA-wide synchronisation: its release at GPU scope is cumulative over what the
 // other threads of the CTA wrote before that synchronisation.  One thread waits for the promotion warps, which meet
 // again behind it; the TMA producer waits with its whole warp.

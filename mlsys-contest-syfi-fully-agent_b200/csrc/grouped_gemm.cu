@@ -69,11 +69,6 @@ struct Cfg {
   // 128-token tiles run un-swapped: tokens are the UMMA M operand (TMEM lanes), weight rows the N operand
   // (TMEM columns).  A promotion thread then owns one token row, so the scale product of a K-block is ONE
   // value per thread instead of one per token column, and the result row is contiguous in memory.
-  // UMMA issuer threads (warps 1 and 2 of the control warpgroup), taking alternate stages.  A stage's UMMAs only
-  // touch that stage's shared memory and TMEM columns and each thread commits its own, so stages are independent;
-  // with one thread the waits and loop overhead between two stages (~500 cycles) leave the tensor pipe idle,
-  // because the instruction queue behind the issuing thread is only an instruction or two deep.
-  static constexpr int ISSUERS = N_TILE >= 32 ? 2 : 1;
   static constexpr bool TOK_ON_M = N_TILE == 128 && GEMM == 1;   // (GEMM2 measures the same either way)
   // Ragged token tiles (swapped orientation only): an item brings and multiplies the rows it has, rounded up to
   // RSTEP.  An SM takes in about 45 bytes per clock from L2 and HBM delivers a 16 KB weight tile every ~700
@@ -208,7 +203,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
   if (warp < kFirstEpiWarp) {
     bool ok = true;
     if (warp == 0) {
-      // ---------------------------------------------------------------- TMA producer (lane 0 issues)
+      // ---------------------------------------------------------------- TMA producer (an elected lane issues)
       for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
         const Item w = decode_item<GEMM, N_TILE>(i, split, ls);
         const int wy = w.e * C::M_TOTAL + w.m * 128;
@@ -253,8 +248,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
           advance();
         }
       }
-    } else if (warp <= C::ISSUERS) {
-      // ---------------------------------------------------------------- UMMA issuer(s) (lane 0 issues)
+    } else {
+      // ---------------------------------------------------------------- UMMA issuers (warps 1 and 2, an elected lane issues)
+      // They take alternate stages.  A stage's UMMAs only touch that stage's shared memory and TMEM columns and each issuer
+      // commits its own, so stages are independent; with one issuer the waits and loop overhead between two stages
+      // (~500 cycles) leave the tensor pipe idle, because the queue behind it is only an instruction or two deep.
       const uint64_t desc_const = umma_desc_k_sw128(0);          // everything but the start address
       int nst = 0;
       for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
@@ -262,7 +260,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
         const uint32_t idesc = umma_idesc_e4m3(128, C::STACK ? C::NTERMS * w.nv : w.nv);
         const uint32_t plane_bytes = static_cast<uint32_t>(w.nv) * 128;
         for (int kb = w.kb0; kb < w.kb1; kb += C::KPS, ++nst, advance()) {   // items span whole stages
-          if (C::ISSUERS == 2 && (nst & 1) != warp - 1) continue;             // the other issuer's stage
+          if ((nst & 1) != warp - 1) continue;             // the other issuer's stage
           if (!mbar_wait(tempty_base + buf * 8, bph ^ 1u, abort_flag)) { ok = false; break; }
           if (!mbar_wait(full_base + stage * 8, ph, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
@@ -330,42 +328,39 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_const
             fma_scaled<C::CPW>(acc, v, f);
           }
         } else {
-          // Every partial of the stage is read back (GB K-blocks at a time, as many as the registers hold) before the
-          // buffer is released and the arithmetic starts.  The stacked planes are w.nv columns apart.  A warp whose
-          // columns start past the item's rows reads nothing (they are never stored).
-          constexpr int GB = C::G * C::PLANES * C::CPW <= 96 ? C::G : 1;
+          // Every partial of the stage is read back before the buffer is released and the arithmetic starts.  The
+          // stacked planes are w.nv columns apart.  A warp whose columns start past the item's rows reads nothing (they
+          // are never stored).
+          static_assert(C::G * C::PLANES * C::CPW <= 96, "the partials of a stage must fit the registers");
           const bool live = h * C::CPW < w.nv;
+          float v[C::G][C::PLANES][C::CPW];
+          if (live) {
 #pragma unroll
-          for (int g0 = 0; g0 < C::G; g0 += GB) {
-            float v[GB][C::PLANES][C::CPW];
-            if (live) {
+            for (int g = 0; g < C::G; ++g)
 #pragma unroll
-              for (int g = 0; g < GB; ++g)
+              for (int p = 0; p < C::PLANES; ++p) tmem_ld_cols<C::CPW>(taddr + g * C::KB_COLS + p * w.nv, v[g][p]);
+            tmem_wait_ld();
+          }
+          release();
+          if (!live) continue;
 #pragma unroll
-                for (int p = 0; p < C::PLANES; ++p) tmem_ld_cols<C::CPW>(taddr + (g0 + g) * C::KB_COLS + p * w.nv, v[g][p]);
-              tmem_wait_ld();
-            }
-            if (g0 + GB == C::G) release();
-            if (!live) continue;
+          for (int g = 0; g < C::G; ++g) {
+            const float ws = sl[C::KPS * N_TILE + g];
+            const float4* scv = reinterpret_cast<const float4*>(sl + g * N_TILE + h * C::CPW);
 #pragma unroll
-            for (int g = 0; g < GB; ++g) {
-              const float ws = sl[C::KPS * N_TILE + g0 + g];
-              const float4* scv = reinterpret_cast<const float4*>(sl + (g0 + g) * N_TILE + h * C::CPW);
+            for (int u = 0; u < C::CPW / 4; ++u) {
+              const float4 f = scv[u];
+              const float2 f2[2] = {__fmul2_rn(make_float2(f.x, f.y), make_float2(ws, ws)),
+                                    __fmul2_rn(make_float2(f.z, f.w), make_float2(ws, ws))};
 #pragma unroll
-              for (int u = 0; u < C::CPW / 4; ++u) {
-                const float4 f = scv[u];
-                const float2 f2[2] = {__fmul2_rn(make_float2(f.x, f.y), make_float2(ws, ws)),
-                                      __fmul2_rn(make_float2(f.z, f.w), make_float2(ws, ws))};
+              for (int x = 0; x < 2; ++x) {
+                const int c = u * 4 + 2 * x;
+                float2 sum = make_float2(v[g][C::PLANES - 1][c], v[g][C::PLANES - 1][c + 1]);
 #pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                  const int c = u * 4 + 2 * x;
-                  float2 sum = make_float2(v[g][C::PLANES - 1][c], v[g][C::PLANES - 1][c + 1]);
-#pragma unroll
-                  for (int p = C::PLANES - 2; p >= 0; --p) sum = __fadd2_rn(sum, make_float2(v[g][p][c], v[g][p][c + 1]));   // smallest terms first
-                  const float2 r = __ffma2_rn(sum, f2[x], make_float2(acc[c], acc[c + 1]));
-                  acc[c] = r.x;
-                  acc[c + 1] = r.y;
-                }
+                for (int p = C::PLANES - 2; p >= 0; --p) sum = __fadd2_rn(sum, make_float2(v[g][p][c], v[g][p][c + 1]));   // smallest terms first
+                const float2 r = __ffma2_rn(sum, f2[x], make_float2(acc[c], acc[c + 1]));
+                acc[c] = r.x;
+                acc[c + 1] = r.y;
               }
             }
           }
