@@ -238,12 +238,10 @@ def test_fused_large_batch_path_against_unfused_path(pkg, dev, W, options, T, se
     assert m["cosine"] >= 0.999999 and m["match_ratio"] == 1.0
 
 
-@pytest.mark.parametrize("counts", [[1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160], [255, 256, 257, 1]])
-def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, counts):
-    """Experts whose row counts sit at the edges of the 32-row steps and of the 128-token tiles: every token with work
-    selects exactly one local expert, `counts[e]` tokens expert e, and the batch is filled up with tokens that have
-    none.  Same bars as every other batch against the oracle."""
-    T = max(1100, sum(counts) + 5)
+def check_rows_per_expert(pkg, dev, W, T, counts):
+    """A batch of T tokens in which expert e of the shard gets exactly `counts[e]` rows and no other expert any: the first
+    sum(counts) tokens select one local expert each, the others none.  Same bars as every other batch against the
+    oracle; that the batch is what it is meant to be is checked on the oracle's and on the operator's side."""
     tok = pkg.gen.make_tokens(T, 11, dev)
     logits = tok.routing_logits * 0.01 - 6.0
     logits[:, 32:35] += 12.0                      # seven experts of groups 1 to 3 for everybody
@@ -255,11 +253,36 @@ def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, counts):
     bias = torch.zeros_like(tok.routing_bias)
     ref = moe_oracle.run_full(logits, bias, tok.hidden_states, tok.hidden_states_scale, W.gemm1_weights,
                               W.gemm1_weights_scale, W.gemm2_weights, W.gemm2_weights_scale, 0, RSF)
+    want = counts + [0] * (32 - len(counts))
+    assert ref.counts.tolist() == want
     out = pkg.op.run(logits, bias, tok.hidden_states, tok.hidden_states_scale, W.gemm1_weights, W.gemm1_weights_scale,
                      W.gemm2_weights, W.gemm2_weights_scale, 0, RSF)
     assert pkg.op.kernel_status() == 0
+    assert list(pkg.op.read_schedule(T).counts) == want
     assert_output_close(out, ref.output, ref.output_f32)
     assert float(out[sum(counts):].float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("fast_combine", [False, True])
+@pytest.mark.parametrize("counts", [[1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160], [255, 256, 257, 1]])
+def test_ragged_token_tiles_of_the_large_batch_path(pkg, dev, W, options, counts, fast_combine):
+    """Experts whose row counts sit at the edges of the 32-row steps and of the 128-token tiles, with both combines."""
+    options(pkg.loader.OPT_FAST_COMBINE if fast_combine else 0)
+    check_rows_per_expert(pkg, dev, W, max(1100, sum(counts) + 5), counts)
+
+
+@pytest.mark.parametrize("T,counts", [
+    (30, [1, 15]), (30, [16, 2, 8]), (32, [17, 14]),                   # 32-token tiles in both GEMMs, one launch routes
+    (64, [1, 15, 16, 17]), (64, [31, 32]), (60, [48, 7]), (64, [49, 1]),   # GEMM1 on 64-token tiles, GEMM2 on 32
+    (200, [1, 15, 16, 17, 31, 32, 33]), (200, [47, 48, 49]),          # 32 / 32 with several tiles an expert
+    (700, [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 113]),  # 64 / 32
+    (900, [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 127, 128, 129]),   # 64 / 64
+])
+def test_ragged_token_tiles_up_to_1024_tokens(pkg, dev, W, T, counts):
+    """Experts whose row counts sit at the edges of the 16-row steps and of the 32- and 64-token tiles of the multi-kernel
+    path, where the number of rows an item brings sets the distance of GEMM2's planes in TMEM, which scales are copied
+    and which promotion warps read nothing."""
+    check_rows_per_expert(pkg, dev, W, T, counts)
 
 
 @pytest.mark.parametrize("T,seed,skew,offset", [(4096, 0, False, 0), (1100, 3, True, 0), (6000, 5, False, 96)])
