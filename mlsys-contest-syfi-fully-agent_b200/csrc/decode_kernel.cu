@@ -576,10 +576,10 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__
 
   tc_fence_before_sync();
   __syncthreads();
-  if (aux->abort) settle_after_abort();
   if (threadIdx.x == 0 && aux->abort) atomicOr(&sched->status, kErrGemm1Timeout | kErrGemm2Timeout);
   if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<volatile unsigned int*>(epoch) = call_tag;   // the next launch's tag differs
   if (warp == 1) {
+    if (aux->abort) settle_after_abort();
     __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, DC::TMEM_COLS);

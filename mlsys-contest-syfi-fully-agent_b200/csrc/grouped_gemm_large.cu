@@ -449,9 +449,9 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
 
   tc_fence_before_sync();
   __syncthreads();
-  if (aux->abort) settle_after_abort();
   if (threadIdx.x == 0 && aux->abort) atomicOr(&sched->status, GEMM == 1 ? kErrGemm1Timeout : kErrGemm2Timeout);
   if (warp == 1) {
+    if (aux->abort) settle_after_abort();
     __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, C::TMEM_COLS);

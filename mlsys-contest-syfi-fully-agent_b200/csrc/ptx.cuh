@@ -115,6 +115,7 @@ __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
 // in flight, and they write shared memory and TMEM that belong to somebody else once it has left.  The barriers they
 // report to can be half armed (a role that left early has not arrived), so this waits for time and not for them:
 // MOE_ABORT_SETTLE_NS, hundreds of times what a load or a stage of UMMAs takes.
+// The warp that frees the TMEM does it; it keeps the CTA's shared memory as well.
 #ifndef MOE_ABORT_SETTLE_NS
 #define MOE_ABORT_SETTLE_NS 1000000ull
 #endif
