@@ -211,6 +211,63 @@ def wtuple(w):
     return (w.gemm1_weights, w.gemm1_weights_scale, w.gemm2_weights, w.gemm2_weights_scale)
 
 
+LINE_LIMIT = 4000              # characters; a reader that keeps the tail of the output still gets the whole line
+
+
+def _short(x):
+    """Floats at six significant digits (ratios close to one at nine), all the way down."""
+    if isinstance(x, float):
+        return float(f"{x:.9g}" if 0.99 < x < 1.0 else f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: _short(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_short(v) for v in x]
+    return x
+
+
+def _row(r):
+    """A sweep row in the line: time, rate, the two roofline fractions of the operator, the slower kernel's, parity."""
+    out = {"workload": r["workload"], "us": r["us_per_step"], "tokens_per_s": r["tokens_per_s"],
+           "hbm_frac": r["whole_op"]["hbm"]["frac"], "fp8_frac": r["whole_op"]["fp8"]["frac"],
+           "kernel": r["roofline"]["kernel"].split(":")[0], "kernel_frac": r["roofline"]["frac"],
+           "cosine": r["parity"]["cosine"], "match_ratio": r["parity"]["match_ratio"]}
+    out.update({k: True for k, v in r["options"].items() if v})
+    return out
+
+
+def compact(line):
+    """The line that is printed: everything that describes the measured workload, and of the other workloads, the ranks
+    and the stages what fits LINE_LIMIT."""
+    out = dict(line)
+    for k in ("sweep", "sweep_modes"):
+        if k in out:
+            out[k] = [_row(r) for r in out[k]]
+    if "scale_anchor" in out:
+        a = out["scale_anchor"]
+        out["scale_anchor"] = {k: a[k] for k in ("workload", "ms_per_step", "tokens_per_s", "records")}
+        out["scale_anchor"].update({k: a["parity"][k] for k in ("cosine", "match_ratio")})
+    if "oracle_vs_oracle" in out:
+        out["oracle_vs_oracle"] = {k: out["oracle_vs_oracle"][k] for k in ("max_abs_over_rms", "n", "n_diff")}
+    if "reference_cuda" in out and "unavailable" not in out["reference_cuda"]:
+        out["reference_cuda"] = {n: r["us_per_step"] for n, r in out["reference_cuda"].items()}
+    for k in ("kernels", "parity_per_rank"):      # whole: only in the full rows
+        out.pop(k, None)
+    out = _short(out)
+    for k in ("oracle_vs_oracle", "run_info", "whole_op", "stage_us", "sweep_modes", "per_gpu"):   # least needed first
+        if len(json.dumps(out)) <= LINE_LIMIT:
+            break
+        out.pop(k, None)
+    return out
+
+
+def emit(line, detail=None):
+    """Prints the one JSON line; `detail`: a file that gets every row in full."""
+    if detail:
+        with open(detail, "w") as f:
+            json.dump(line, f)
+    print(json.dumps(compact(line)), flush=True)
+
+
 def workload_config(name, n_sel, n_active):
     """The `config` block of a single-GPU line; both arms print exactly this."""
     wl = WORKLOADS[name]
@@ -502,7 +559,7 @@ def bench_single(args):
         ours.update({r["workload"]: r["us_per_step"] for r in rows})
         if "unavailable" not in ref_rows:
             line["speedup_vs_reference_cuda"] = {n: ref_rows[n]["us_per_step"] / ours[n] for n in ours if n in ref_rows}
-    print(json.dumps(line))
+    emit(line, args.detail)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -757,7 +814,7 @@ def bench_ep(args):
         else:
             dom = None
         per = 8 // world
-        print(json.dumps({
+        emit({
             "metric": METRIC, "value": EP_T / (ms_step * 1e-3), "unit": UNIT,
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
             "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "fp8_e4m3",
@@ -791,7 +848,7 @@ def bench_ep(args):
             "parity": merge_parity(reports),
             "parity_per_rank": reports,
             "cpu_baseline": None,
-        }))
+        }, args.detail)
     if world > 1:
         dist.destroy_process_group()
 
@@ -1012,6 +1069,8 @@ def main():
     ap.add_argument("--profile-only", action="store_true",
                     help="run W + K steps of the workload and exit (no checks, no CPU legs): the command profiler "
                          "captures are taken from")
+    ap.add_argument("--detail", default=None, metavar="FILE",
+                    help="also write every row in full (all stages, rooflines and parity numbers of the sweep) to FILE")
     ap.add_argument("--replay", default=None, metavar="ROOT",
                     help="replay a flashinfer-trace workload set rooted at ROOT ('synthetic': a stand-in set written to "
                          "a temporary directory) and print the per-workload table")
