@@ -7,9 +7,10 @@
 
 namespace moe {
 
-// Three warpgroups: warpgroup 0 holds the TMA producer (warp 0) and the UMMA issuer (warp 1) and gives
-// most of its registers away (setmaxnreg); warpgroups 1 and 2 are the eight promotion / epilogue warps
-// (warp % 4 = the TMEM lane quarter a warp may access) and take them.
+// Three warpgroups: warpgroup 0 holds the TMA producer (warp 0) and the UMMA issuer (warp 1; grouped GEMM: warps 1 and 2,
+// and the scale warp 3), warpgroups 1 and 2 are the eight promotion / epilogue warps (warp % 4 = the TMEM lane quarter a
+// warp may access).  In the decode kernel warpgroup 0 gives most of its registers away (setmaxnreg) and the others take
+// them; the grouped GEMM leaves every thread its share.
 constexpr int kEpiWarps = 8;
 constexpr int kFirstEpiWarp = 4;
 constexpr int kGemmThreads = (kFirstEpiWarp + kEpiWarps) * 32;
@@ -22,8 +23,8 @@ static_assert(128 * kRegsControl + 256 * kRegsEpilogue <= kRegsAtLaunch * kGemmT
 static_assert(kRegsControl % 8 == 0 && kRegsEpilogue % 8 == 0, "setmaxnreg takes multiples of 8");
 
 struct Aux {
-  uint64_t full[10];       // TMA -> issuer: the stage's operands have landed
-  uint64_t done[10];       // issuer -> producer and promotion warps: the stage's UMMAs have completed
+  uint64_t full[10];       // TMA (and scale warp) -> issuer: the stage's operands have landed
+  uint64_t done[10];       // issuer -> producer, scale and promotion warps: the stage's UMMAs have completed
   uint64_t tempty[4];      // promotion warps -> issuer: the TMEM buffer has been read
   uint64_t esync;          // bounded replacement for a named barrier among the epilogue threads
   uint32_t tmem_base;

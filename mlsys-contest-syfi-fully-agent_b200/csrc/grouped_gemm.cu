@@ -15,7 +15,7 @@
 //   warp 0  producer: TMA (SWIZZLE_128B, no multicast) of one weight tile
 //           [128 rows x 128 K-bytes] and the token tile(s) [N_TILE x 128] per K-block
 //           into a ring of STAGES shared-memory stages.
-//   warps 1, 2  issuers (alternate stages): one lane issues the tcgen05.mma kind::f8f6f4 (M128, K32) of a
+//   warps 1, 2  issuers (alternate stages): an elected lane issues the tcgen05.mma kind::f8f6f4 (M128, K32) of a
 //           K-block into its own TMEM columns.  For GEMM2 the kNTerms e4m3 planes of
 //           the token operand sit back to back in shared memory and, while they fit
 //           N <= 256, are consumed as ONE operand of N = kNTerms * N_TILE rows, so the
@@ -24,12 +24,11 @@
 //           NBUF groups rotate through TMEM so that the hand-off latency between the
 //           tensor core and the promotion warps is hidden.
 //   warp 3  scales of every stage, copied asynchronously (cp.async) into a ring of slots behind the stage's own
-//           "full" barrier, so that the promotion warps never wait for global memory.  They used to build a table
-//           of scale products per item, and decoded the item by a binary search in shared memory: 3000 to 7000
-//           clocks per item without a UMMA in flight, a third of GEMM2 at T = 512.  With this, and one elected lane
-//           instead of `lane == 0` around the UMMAs and TMA loads (ptx.cuh), a call at T = 512 takes 248 instead of
-//           265 us, at T = 901 304 instead of 331, at T = 64 with all rows on 16 experts 176 instead of 189
-//           (sustained load, power-capped clocks; 230, 275, 168 instead of 249, 306, 181 on a cool GPU).
+//           "full" barrier, so that the promotion warps never wait for global memory.  Visible to them because the
+//           issuer, which waited on "full", arrives on the stage's "done" barrier beside its commit.  A table of
+//           scale products built by the promotion warps per item instead left 3000 to 7000 clocks per item without
+//           a UMMA in flight, a third of GEMM2 at T = 512 (without it, and with the elected issue and the packed
+//           arithmetic, calls are 1.07 times as fast at T = 512, 1.09 at T = 901, 1.08 at T = 64 on 16 experts).
 //   warps 4-11 promotion + epilogue (two warps per TMEM lane quarter, each owning half
 //           of the token columns): tcgen05.ld the partials of a group, release the TMEM
 //           buffer, multiply by w_scale[e, m, kb] * b_scale[row, kb] and accumulate in
@@ -71,9 +70,9 @@ struct Cfg {
   // value per thread instead of one per token column, and the result row is contiguous in memory.
   static constexpr bool TOK_ON_M = N_TILE == 128 && GEMM == 1;   // (GEMM2 measures the same either way)
   // Ragged token tiles (swapped orientation only): an item brings and multiplies the rows it has, rounded up to
-  // RSTEP.  An SM takes in about 45 bytes per clock from L2 and HBM delivers a 16 KB weight tile every ~700
-  // clocks per SM, so a K-block may cost 31 KB of operands before the weight stream stalls; GEMM2's three
-  // planes of a full 64-token tile alone are 24 KB.
+  // RSTEP.  An SM takes in about 51 bytes per clock (large-batch GEMM1 at T = 4096 without its promotion: 48 KB K-blocks
+  // in 962 clocks) and HBM delivers a 16 KB weight tile every ~700 clocks per SM, so a K-block may cost 35 KB of
+  // operands before the weight stream stalls; with GEMM2's three planes a full 64-token tile makes it 40 KB.
   static constexpr int RSTEP = N_TILE >= 64 ? N_TILE / 4 : 16;
   static constexpr int RMAPS = N_TILE / RSTEP;
   static_assert(RMAPS >= 1 && RMAPS <= 4 && RSTEP % 16 == 0, "token maps per kernel / UMMA N granularity");

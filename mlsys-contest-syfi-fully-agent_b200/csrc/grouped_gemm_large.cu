@@ -10,7 +10,8 @@
 //     C = silu(x2) * x1 (full-agent-pipeline/references/moe.py:187-193: the SECOND half goes through
 //     silu) of its token row, the four threads of a row agree on the block's power-of-two scale, and C
 //     goes out as the three e4m3 planes + scale that GEMM2 reads.  The wide tile is also what the
-//     hardware wants: an SM takes in about 45 bytes per clock from L2, a 128 x 128 x 128 fp8 tile needs
+//     hardware wants: an SM takes in about 51 bytes per clock (48 KB K-blocks in 962 clocks at T = 4096,
+//     without the promotion), a 128 x 128 x 128 fp8 tile needs
 //     32 KB per 256 tensor-pipe clocks (128 B / clock), a 128 x 256 tile 48 KB per 512 (96 B / clock).
 //   GEMM2 (+ combine):  replaces gemm_fp32_fp8w_fused_acc_grouped_kernel and fin_cast8_kernel
 //     (moe.cu:2186-2431, 2473-2496).  COMBINE = false stores fp32 rows for the deterministic
@@ -41,7 +42,8 @@
 //               latency of one warp is covered by the FMAs of the others; with eight the read-back
 //               latency was exposed in every K-block and the tensor pipe sat idle two thirds of the time.
 // The two rings, the scale warp, the ragged boxes and the elected lanes together: T = 4096 778 -> 695 us per call,
-// T = 14107 1644 -> 1475 us, the 256-expert layer at T = 16384 15.3 -> 13.9 ms (per call, both builds in turn).
+// T = 14107 1644 -> 1475 us, the 256-expert layer at T = 16384 15.3 -> 13.9 ms (per call, both builds in turn; the
+// kernels alone at T = 4096: GEMM1 341 -> 279 us, GEMM2 288 -> 252).
 // Every wait is bounded (ptx.cuh); a timeout raises the CTA's abort flag, all roles fall through to
 // the normal teardown (TMEM freed) and an error bit is left in the schedule block.
 #include "epilogue_device.cuh"

@@ -130,14 +130,15 @@ int route_permute_launches(int T);   // kernels launch_route_permute starts for 
 void launch_route_permute(const RouteArgs& r, const PermuteArgs& p, cudaStream_t stream);
 void launch_route_only(const RouteArgs& r, cudaStream_t stream);
 void launch_gather_rows(const GatherArgs& a, int T, cudaStream_t stream);
-// gemm_id 1 or 2; n_tile in {32, 64, 128}.  Returns a cudaError_t as int.
-// Token-operand tensor maps of the grouped GEMM kernels: the same tensor with boxes of 1..4 row steps, so that a token tile with few valid rows (the last tile of an
-// expert, or an expert with a handful of tokens) brings only the rows it has, rounded up to a step.
+// Token-operand tensor maps of the grouped GEMM kernels: the same tensor with boxes of 1..4 row steps, so that a token
+// tile with few valid rows (the last tile of an expert, or an expert with a handful of tokens) brings only the rows it
+// has, rounded up to a step.
 struct TokenMaps {
   CUtensorMap m[4];
 };
 int grouped_gemm_row_step(int n_tile);
 constexpr int kLargeRowStep = 32;   // row step of the large-batch kernels (one TMEM lane quarter)
+// gemm_id 1 or 2; n_tile in {32, 64, 128}.  Returns a cudaError_t as int.
 int launch_grouped_gemm(int gemm_id, int n_tile, const CUtensorMap& tm_w, const TokenMaps& tm_b, const GemmArgs& a,
                         int ctas, cudaStream_t stream);
 constexpr int kFusedMaxTokens = 16;

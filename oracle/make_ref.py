@@ -31,7 +31,8 @@ import subprocess
 HERE = os.path.dirname(os.path.abspath(__file__))
 DEST_DIR = os.path.join(HERE, "_ref")
 DEST = os.path.join(DEST_DIR, "moe_definition.py")
-DEFAULT_REFERENCE = os.environ.get("MOE_REFERENCE_ROOT", "/root/reference")   # checkout of the reference repository
+# checkout of the reference repository: beside this repository unless the environment names it
+DEFAULT_REFERENCE = os.environ.get("MOE_REFERENCE_ROOT", os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference"))
 
 
 def make_ref(reference: str = DEFAULT_REFERENCE):
