@@ -218,7 +218,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
 #pragma unroll 1
         for (int kb = 0; kb < C::KB; ++kb, ++n, wp.step()) {
           if (n >= C::WS) {
-            if (!mbar_wait(pdone_base + old.i * 8, old.ph, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_hot(pdone_base + old.i * 8, old.ph, abort_flag)) { ok = false; break; }
             old.step(C::NTERMS);
           }
           if (elect_one()) {
@@ -240,7 +240,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
             pp.step();
           } else {
             for (int t = 0; t < C::NTERMS; ++t, pp.step()) {
-              if (!mbar_wait(pdone_base + pp.i * 8, pp.ph ^ 1u, abort_flag)) { ok = false; break; }
+              if (!mbar_wait_hot(pdone_base + pp.i * 8, pp.ph ^ 1u, abort_flag)) { ok = false; break; }
               if (elect_one()) {
                 const uint32_t bar = pfull_base + pp.i * 8;
                 mbar_arrive_expect_tx(bar, tok_tx);
@@ -264,7 +264,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
 #pragma unroll 1
         for (int kb = 0; kb < C::KB; ++kb, ++n, wp.step()) {
           if (n >= C::WS) {
-            if (!mbar_wait(pdone_base + old.i * 8, old.ph, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_hot(pdone_base + old.i * 8, old.ph, abort_flag)) { ok = false; break; }
             old.step(C::NTERMS);
           }
           const float* bsp = a.b_scale + static_cast<size_t>(kb) * a.rows_cap;
@@ -287,14 +287,14 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
 #pragma unroll 1
         for (int s = 0; s < C::KB; ++s, ++n) {
           if ((n & 1) == warp - 1) {
-            if (!mbar_wait(tempty_base + tb.i * 8, tb.ph ^ 1u, abort_flag)) { ok = false; break; }
-            if (!mbar_wait(wfull_base + wp.i * 8, wp.ph, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_hot(tempty_base + tb.i * 8, tb.ph ^ 1u, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_hot(wfull_base + wp.i * 8, wp.ph, abort_flag)) { ok = false; break; }
             const uint64_t wdesc = desc_const | ((smem_base + wp.i * C::W_BYTES) >> 4);
             const uint32_t d = tmem_base + tb.i * C::BUF_COLS;
 #pragma unroll
             for (int t = 0; t < C::NTERMS; ++t, pp.step()) {
               if constexpr (!JOINT) {
-                if (!mbar_wait(pfull_base + pp.i * 8, pp.ph, abort_flag)) { ok = false; break; }
+                if (!mbar_wait_hot(pfull_base + pp.i * 8, pp.ph, abort_flag)) { ok = false; break; }
               }
               tc_fence_after_sync();
               if (elect_one()) {
@@ -338,7 +338,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
     bool ok = true;
     auto epi_sync = [&]() {
       mbar_arrive(smem_u32(&aux->esync));
-      if (!mbar_wait(smem_u32(&aux->esync), eph, abort_flag)) ok = false;
+      if (!mbar_wait_hot(smem_u32(&aux->esync), eph, abort_flag)) ok = false;
       eph ^= 1u;
     };
     for (int i = blockIdx.x; ok && i < items; i += gridDim.x) {
@@ -350,7 +350,7 @@ grouped_gemm_large_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       const bool live = q * 32 < w.valid;         // a warp whose rows lie past the tile's last one reads nothing
 #pragma unroll 1
       for (int s = 0; s < C::KB; ++s, last.step(C::NTERMS), tb.step()) {
-        if (!mbar_wait(pdone_base + last.i * 8, last.ph, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_hot(pdone_base + last.i * 8, last.ph, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
         const float* sl = slots + slot * C::SLOT_FLOATS;
         if (++slot == C::NSLOT) slot = 0;
